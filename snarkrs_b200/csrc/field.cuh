@@ -7,18 +7,18 @@
 // bit with the CPU prover.
 //
 // The Montgomery product is CIOS (Koc, Acar and Kaliski, "Analyzing and
-// comparing Montgomery multiplication algorithms", 1996) in two forms with
-// identical results:
-//   * mul_cc: PTX multiply-add carry chains -- per limb of b, one
-//     mad.lo.cc/madc.lo.cc chain and one mad.hi.cc/madc.hi.cc chain for
-//     a*b[i], then the same pair for m*p, each chain in one asm statement.
-//     Used by the NTT butterflies.
-//   * mul: the same CIOS on 32x32->64-bit multiply-adds with the carries in
-//     64-bit sums, which the compiler lowers to wide IMADs plus 3-input adds
-//     on the ALU pipe.  On sm_100a it measured 843 cycles for one warp's
-//     dependent product against 1381 for mul_cc, 45.8 against 43.7 G
-//     products/s at full occupancy, and 5-38% faster MSM kernels, so every
-//     point formula uses it.
+// comparing Montgomery multiplication algorithms", 1996) with the running sum
+// held as two vectors of 64-bit lanes, one over the even limb positions and
+// one over the odd ones (the column split that Emmart, Zheng and Weems use on
+// GPUs).  Within a vector the partial products a[j] b do not overlap, so a row
+// is one carry chain of 32x32+64-bit multiply-adds and no other instruction;
+// the carry between the vectors rides into the next row's chain.  What bounds
+// it is the issue rate of wide multiply-adds, 32 a clock on an SM: 136 of them
+// a product leave 69.6 G products/s on 148 SMs at 1965 MHz, and it measured
+// 66.5 G/s (one product per thread and step, 1024 threads an SM) and 845
+// cycles for one warp's dependent product, against 44.0 G/s and 1127 cycles
+// for the form it replaced, a single vector whose carries were 64-bit sums on
+// the ALU pipe.
 // BN254's moduli are below 2^254, so the running sum stays below 2^287 and
 // fits nine limbs; the carry out of the ninth is provably zero.
 #pragma once
@@ -181,198 +181,429 @@ __device__ __forceinline__ Fp<Params> dbl(const Fp<Params>& a) {
     return add(a, a);
 }
 
-// t[0..8] += a[0..7] * b  (lo halves into t0..t7 with carry into t8, then hi halves into t1..t8)
-#define G16_MAD_ROW(T, A, B)                                                                         \
-    asm("mad.lo.cc.u32  %0, %9, %17, %0;\n\t"                                                        \
-        "madc.lo.cc.u32 %1, %10, %17, %1;\n\t"                                                       \
-        "madc.lo.cc.u32 %2, %11, %17, %2;\n\t"                                                       \
-        "madc.lo.cc.u32 %3, %12, %17, %3;\n\t"                                                       \
-        "madc.lo.cc.u32 %4, %13, %17, %4;\n\t"                                                       \
-        "madc.lo.cc.u32 %5, %14, %17, %5;\n\t"                                                       \
-        "madc.lo.cc.u32 %6, %15, %17, %6;\n\t"                                                       \
-        "madc.lo.cc.u32 %7, %16, %17, %7;\n\t"                                                       \
-        "addc.u32       %8, %8, 0;\n\t"                                                              \
-        "mad.hi.cc.u32  %1, %9, %17, %1;\n\t"                                                        \
-        "madc.hi.cc.u32 %2, %10, %17, %2;\n\t"                                                       \
-        "madc.hi.cc.u32 %3, %11, %17, %3;\n\t"                                                       \
-        "madc.hi.cc.u32 %4, %12, %17, %4;\n\t"                                                       \
-        "madc.hi.cc.u32 %5, %13, %17, %5;\n\t"                                                       \
-        "madc.hi.cc.u32 %6, %14, %17, %6;\n\t"                                                       \
-        "madc.hi.cc.u32 %7, %15, %17, %7;\n\t"                                                       \
-        "madc.hi.u32    %8, %16, %17, %8;"                                                           \
-        : "+r"(T[0]), "+r"(T[1]), "+r"(T[2]), "+r"(T[3]), "+r"(T[4]), "+r"(T[5]), "+r"(T[6]),        \
-          "+r"(T[7]), "+r"(T[8])                                                                     \
-        : "r"(A[0]), "r"(A[1]), "r"(A[2]), "r"(A[3]), "r"(A[4]), "r"(A[5]), "r"(A[6]), "r"(A[7]),    \
-          "r"(B))
-
-// t[0..8] += m * P, then shift down one limb
-#define G16_REDUCE_ROW(T, M, PP)                                                                     \
-    asm("mad.lo.cc.u32  %0, %9, %10, %0;\n\t"                                                        \
-        "madc.lo.cc.u32 %1, %9, %11, %1;\n\t"                                                        \
-        "madc.lo.cc.u32 %2, %9, %12, %2;\n\t"                                                        \
-        "madc.lo.cc.u32 %3, %9, %13, %3;\n\t"                                                        \
-        "madc.lo.cc.u32 %4, %9, %14, %4;\n\t"                                                        \
-        "madc.lo.cc.u32 %5, %9, %15, %5;\n\t"                                                        \
-        "madc.lo.cc.u32 %6, %9, %16, %6;\n\t"                                                        \
-        "madc.lo.cc.u32 %7, %9, %17, %7;\n\t"                                                        \
-        "addc.u32       %8, %8, 0;\n\t"                                                              \
-        "mad.hi.cc.u32  %1, %9, %10, %1;\n\t"                                                        \
-        "madc.hi.cc.u32 %2, %9, %11, %2;\n\t"                                                        \
-        "madc.hi.cc.u32 %3, %9, %12, %3;\n\t"                                                        \
-        "madc.hi.cc.u32 %4, %9, %13, %4;\n\t"                                                        \
-        "madc.hi.cc.u32 %5, %9, %14, %5;\n\t"                                                        \
-        "madc.hi.cc.u32 %6, %9, %15, %6;\n\t"                                                        \
-        "madc.hi.cc.u32 %7, %9, %16, %7;\n\t"                                                        \
-        "madc.hi.u32    %8, %9, %17, %8;"                                                            \
-        : "+r"(T[0]), "+r"(T[1]), "+r"(T[2]), "+r"(T[3]), "+r"(T[4]), "+r"(T[5]), "+r"(T[6]),        \
-          "+r"(T[7]), "+r"(T[8])                                                                     \
-        : "r"(M), "n"(PP::P(0)), "n"(PP::P(1)), "n"(PP::P(2)), "n"(PP::P(3)), "n"(PP::P(4)),         \
-          "n"(PP::P(5)), "n"(PP::P(6)), "n"(PP::P(7)))
-
-template <class Params>
-__device__ __forceinline__ Fp<Params> mul_cc(const Fp<Params>& a, const Fp<Params>& b) {
-    uint32_t t[9];
-#pragma unroll
-    for (int i = 0; i < 9; i++) t[i] = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        G16_MAD_ROW(t, a.v, b.v[i]);
-        uint32_t m = t[0] * Params::N0;
-        G16_REDUCE_ROW(t, m, Params);
-        // t0 is now zero: shift down
-#pragma unroll
-        for (int j = 0; j < 8; j++) t[j] = t[j + 1];
-        t[8] = 0;
+// ---- r = a + b, r = a - b over 8 or 16 words, the last carry or borrow dropped ----
+// (early-clobber outputs: a word of r is written before the later words of a
+// and b are read)
+template <int N>
+__host__ __device__ __forceinline__ void add_words(uint32_t* r, const uint32_t* a, const uint32_t* b) {
+    static_assert(N == 8 || N == 16, "word count");
+#ifdef __CUDA_ARCH__
+    if constexpr (N == 8)
+        asm("add.cc.u32 %0, %8, %16;\n\t"
+            "addc.cc.u32 %1, %9, %17;\n\t"
+            "addc.cc.u32 %2, %10, %18;\n\t"
+            "addc.cc.u32 %3, %11, %19;\n\t"
+            "addc.cc.u32 %4, %12, %20;\n\t"
+            "addc.cc.u32 %5, %13, %21;\n\t"
+            "addc.cc.u32 %6, %14, %22;\n\t"
+            "addc.u32  %7, %15, %23;"
+            : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]),
+              "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]));
+    else
+        asm("add.cc.u32 %0, %16, %32;\n\t"
+            "addc.cc.u32 %1, %17, %33;\n\t"
+            "addc.cc.u32 %2, %18, %34;\n\t"
+            "addc.cc.u32 %3, %19, %35;\n\t"
+            "addc.cc.u32 %4, %20, %36;\n\t"
+            "addc.cc.u32 %5, %21, %37;\n\t"
+            "addc.cc.u32 %6, %22, %38;\n\t"
+            "addc.cc.u32 %7, %23, %39;\n\t"
+            "addc.cc.u32 %8, %24, %40;\n\t"
+            "addc.cc.u32 %9, %25, %41;\n\t"
+            "addc.cc.u32 %10, %26, %42;\n\t"
+            "addc.cc.u32 %11, %27, %43;\n\t"
+            "addc.cc.u32 %12, %28, %44;\n\t"
+            "addc.cc.u32 %13, %29, %45;\n\t"
+            "addc.cc.u32 %14, %30, %46;\n\t"
+            "addc.u32  %15, %31, %47;"
+            : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]),
+          "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(a[8]),
+          "r"(a[9]), "r"(a[10]), "r"(a[11]), "r"(a[12]), "r"(a[13]), "r"(a[14]), "r"(a[15]),
+              "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]), "r"(b[8]),
+          "r"(b[9]), "r"(b[10]), "r"(b[11]), "r"(b[12]), "r"(b[13]), "r"(b[14]), "r"(b[15]));
+#else
+    uint64_t c = 0;
+    for (int k = 0; k < N; k++) {
+        c += (uint64_t)a[k] + b[k];
+        r[k] = (uint32_t)c;
+        c >>= 32;
     }
-    reduce_once<Params>(t);
-    Fp<Params> r;
-#pragma unroll
-    for (int i = 0; i < 8; i++) r.v[i] = t[i];
-    return r;
+#endif
+}
+template <int N>
+__host__ __device__ __forceinline__ void sub_words(uint32_t* r, const uint32_t* a, const uint32_t* b) {
+    static_assert(N == 8 || N == 16, "word count");
+#ifdef __CUDA_ARCH__
+    if constexpr (N == 8)
+        asm("sub.cc.u32 %0, %8, %16;\n\t"
+            "subc.cc.u32 %1, %9, %17;\n\t"
+            "subc.cc.u32 %2, %10, %18;\n\t"
+            "subc.cc.u32 %3, %11, %19;\n\t"
+            "subc.cc.u32 %4, %12, %20;\n\t"
+            "subc.cc.u32 %5, %13, %21;\n\t"
+            "subc.cc.u32 %6, %14, %22;\n\t"
+            "subc.u32  %7, %15, %23;"
+            : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]),
+              "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]));
+    else
+        asm("sub.cc.u32 %0, %16, %32;\n\t"
+            "subc.cc.u32 %1, %17, %33;\n\t"
+            "subc.cc.u32 %2, %18, %34;\n\t"
+            "subc.cc.u32 %3, %19, %35;\n\t"
+            "subc.cc.u32 %4, %20, %36;\n\t"
+            "subc.cc.u32 %5, %21, %37;\n\t"
+            "subc.cc.u32 %6, %22, %38;\n\t"
+            "subc.cc.u32 %7, %23, %39;\n\t"
+            "subc.cc.u32 %8, %24, %40;\n\t"
+            "subc.cc.u32 %9, %25, %41;\n\t"
+            "subc.cc.u32 %10, %26, %42;\n\t"
+            "subc.cc.u32 %11, %27, %43;\n\t"
+            "subc.cc.u32 %12, %28, %44;\n\t"
+            "subc.cc.u32 %13, %29, %45;\n\t"
+            "subc.cc.u32 %14, %30, %46;\n\t"
+            "subc.u32  %15, %31, %47;"
+            : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]),
+          "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(a[8]),
+          "r"(a[9]), "r"(a[10]), "r"(a[11]), "r"(a[12]), "r"(a[13]), "r"(a[14]), "r"(a[15]),
+              "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]), "r"(b[8]),
+          "r"(b[9]), "r"(b[10]), "r"(b[11]), "r"(b[12]), "r"(b[13]), "r"(b[14]), "r"(b[15]));
+#else
+    int64_t c = 0;
+    for (int k = 0; k < N; k++) {
+        c += (int64_t)a[k] - b[k];
+        r[k] = (uint32_t)c;
+        c >>= 32;
+    }
+#endif
 }
 
-// CIOS with 64-bit sums: t[j] + a[j] b[i] + carry < 2^64 always holds
+// ---- rows: N partial products on the 64-bit lanes of x (x[2k], x[2k + 1]) ----
+// A row takes the N words a[0], a[2], .. of its multiplicand (every second
+// one, those that fall on this vector's lanes) times b.  On the device each is
+// one asm statement, since the carry flag does not outlive a statement; the
+// host forms give the same words, for the unit checks of the limbs.
+
+// x = a b
+template <int N>
+__host__ __device__ __forceinline__ void row_mul(uint32_t* x, const uint32_t* a, uint32_t b) {
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const uint64_t p = (uint64_t)a[2 * k] * b;
+        x[2 * k] = (uint32_t)p;
+        x[2 * k + 1] = (uint32_t)(p >> 32);
+    }
+}
+
+#ifndef __CUDA_ARCH__
+// the chain shared by the host forms: x + a b + carry, the carry out returned
+template <int N>
+inline uint32_t row_mad_host(uint32_t* x, const uint32_t* a, uint32_t b, uint32_t carry) {
+    for (int k = 0; k < N; k++) {
+        const uint64_t t = (uint64_t)x[2 * k + 1] << 32 | x[2 * k];
+        const uint64_t p = (uint64_t)a[2 * k] * b, s = t + p, r = s + carry;
+        carry = (uint32_t)(s < t) + (uint32_t)(r < s);
+        x[2 * k] = (uint32_t)r;
+        x[2 * k + 1] = (uint32_t)(r >> 32);
+    }
+    return carry;
+}
+#endif
+
+// x += a b; the caller knows that nothing is carried out of the last lane
+template <int N>
+__host__ __device__ __forceinline__ void row_mad(uint32_t* x, const uint32_t* a, uint32_t b) {
+    static_assert(N >= 1 && N <= 4, "row length");
+#ifdef __CUDA_ARCH__
+    if constexpr (N == 4)
+        asm("mad.lo.cc.u32  %0, %8, %12, %0;\n\t"
+            "madc.hi.cc.u32 %1, %8, %12, %1;\n\t"
+            "madc.lo.cc.u32 %2, %9, %12, %2;\n\t"
+            "madc.hi.cc.u32 %3, %9, %12, %3;\n\t"
+            "madc.lo.cc.u32 %4, %10, %12, %4;\n\t"
+            "madc.hi.cc.u32 %5, %10, %12, %5;\n\t"
+            "madc.lo.cc.u32 %6, %11, %12, %6;\n\t"
+            "madc.hi.u32    %7, %11, %12, %7;"
+            : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7])
+            : "r"(a[0]), "r"(a[2]), "r"(a[4]), "r"(a[6]), "r"(b));
+    else if constexpr (N == 3)
+        asm("mad.lo.cc.u32  %0, %6, %9, %0;\n\t"
+            "madc.hi.cc.u32 %1, %6, %9, %1;\n\t"
+            "madc.lo.cc.u32 %2, %7, %9, %2;\n\t"
+            "madc.hi.cc.u32 %3, %7, %9, %3;\n\t"
+            "madc.lo.cc.u32 %4, %8, %9, %4;\n\t"
+            "madc.hi.u32    %5, %8, %9, %5;"
+            : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5])
+            : "r"(a[0]), "r"(a[2]), "r"(a[4]), "r"(b));
+    else if constexpr (N == 2)
+        asm("mad.lo.cc.u32  %0, %4, %6, %0;\n\t"
+            "madc.hi.cc.u32 %1, %4, %6, %1;\n\t"
+            "madc.lo.cc.u32 %2, %5, %6, %2;\n\t"
+            "madc.hi.u32    %3, %5, %6, %3;"
+            : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3])
+            : "r"(a[0]), "r"(a[2]), "r"(b));
+    else
+        asm("mad.lo.cc.u32  %0, %2, %3, %0;\n\t"
+            "madc.hi.u32    %1, %2, %3, %1;"
+            : "+r"(x[0]), "+r"(x[1])
+            : "r"(a[0]), "r"(b));
+#else
+    row_mad_host<N>(x, a, b, 0);
+#endif
+}
+
+// x += a b, the carry out of the last lane added to c
+template <int N>
+__host__ __device__ __forceinline__ void row_mad_c(uint32_t* x, const uint32_t* a, uint32_t b, uint32_t& c) {
+    static_assert(N >= 1 && N <= 4, "row length");
+#ifdef __CUDA_ARCH__
+    if constexpr (N == 4)
+        asm("mad.lo.cc.u32  %0, %9, %13, %0;\n\t"
+            "madc.hi.cc.u32 %1, %9, %13, %1;\n\t"
+            "madc.lo.cc.u32 %2, %10, %13, %2;\n\t"
+            "madc.hi.cc.u32 %3, %10, %13, %3;\n\t"
+            "madc.lo.cc.u32 %4, %11, %13, %4;\n\t"
+            "madc.hi.cc.u32 %5, %11, %13, %5;\n\t"
+            "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"
+            "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
+            "addc.u32       %8, %8, 0;"
+            : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7]),
+              "+r"(c)
+            : "r"(a[0]), "r"(a[2]), "r"(a[4]), "r"(a[6]), "r"(b));
+    else if constexpr (N == 3)
+        asm("mad.lo.cc.u32  %0, %7, %10, %0;\n\t"
+            "madc.hi.cc.u32 %1, %7, %10, %1;\n\t"
+            "madc.lo.cc.u32 %2, %8, %10, %2;\n\t"
+            "madc.hi.cc.u32 %3, %8, %10, %3;\n\t"
+            "madc.lo.cc.u32 %4, %9, %10, %4;\n\t"
+            "madc.hi.cc.u32 %5, %9, %10, %5;\n\t"
+            "addc.u32       %6, %6, 0;"
+            : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(c)
+            : "r"(a[0]), "r"(a[2]), "r"(a[4]), "r"(b));
+    else if constexpr (N == 2)
+        asm("mad.lo.cc.u32  %0, %5, %7, %0;\n\t"
+            "madc.hi.cc.u32 %1, %5, %7, %1;\n\t"
+            "madc.lo.cc.u32 %2, %6, %7, %2;\n\t"
+            "madc.hi.cc.u32 %3, %6, %7, %3;\n\t"
+            "addc.u32       %4, %4, 0;"
+            : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(c)
+            : "r"(a[0]), "r"(a[2]), "r"(b));
+    else
+        asm("mad.lo.cc.u32  %0, %3, %4, %0;\n\t"
+            "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+            "addc.u32       %2, %2, 0;"
+            : "+r"(x[0]), "+r"(x[1]), "+r"(c)
+            : "r"(a[0]), "r"(b));
+#else
+    c += row_mad_host<N>(x, a, b, 0);
+#endif
+}
+
+// One limb down and the next row: e0 += x[1], and x = (x >> 64) + a b + the
+// carry of that sum.  x holds the even positions of a sum whose lowest limb is
+// zero and e0 is the first odd position; afterwards x holds the odd positions
+// of the sum one limb lower (four lanes) and e0 starts the even ones.
+__host__ __device__ __forceinline__ void row_shift_mad(uint32_t* x, uint32_t& e0, const uint32_t* a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+    asm("add.cc.u32     %8, %8, %1;\n\t"
+        "madc.lo.cc.u32 %0, %9, %13, %2;\n\t"
+        "madc.hi.cc.u32 %1, %9, %13, %3;\n\t"
+        "madc.lo.cc.u32 %2, %10, %13, %4;\n\t"
+        "madc.hi.cc.u32 %3, %10, %13, %5;\n\t"
+        "madc.lo.cc.u32 %4, %11, %13, %6;\n\t"
+        "madc.hi.cc.u32 %5, %11, %13, %7;\n\t"
+        "madc.lo.cc.u32 %6, %12, %13, 0;\n\t"
+        "madc.hi.u32    %7, %12, %13, 0;"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7]), "+r"(e0)
+        : "r"(a[0]), "r"(a[2]), "r"(a[4]), "r"(a[6]), "r"(b));
+#else
+    const uint64_t s = (uint64_t)e0 + x[1];
+    e0 = (uint32_t)s;
+    for (int k = 0; k < 6; k++) x[k] = x[k + 2];
+    x[6] = x[7] = 0;
+    row_mad_host<4>(x, a, b, (uint32_t)(s >> 32));
+#endif
+}
+
+// r = x + y[1..7]: the odd positions of a sum plus its even ones one limb
+// lower (y[0] is zero)
+__host__ __device__ __forceinline__ void merge_odd_even(uint32_t* r, const uint32_t* x, const uint32_t* y) {
+    const uint32_t lower[8] = {y[1], y[2], y[3], y[4], y[5], y[6], y[7], 0};
+    add_words<8>(r, x, lower);
+}
+
+// the modulus' limbs from position i on, as a row's multiplicand
+template <class Params>
+struct Modulus {
+    uint32_t v[8];
+    __host__ __device__ __forceinline__ Modulus() {
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = Params::P(i);
+    }
+};
+
+// even += m p (even limbs), odd += m p (odd limbs), with m chosen so that
+// even[0] becomes zero
+template <class Params>
+__host__ __device__ __forceinline__ void reduce_row(uint32_t* even, uint32_t* odd) {
+    const Modulus<Params> p;
+    const uint32_t m = even[0] * Params::N0;
+    row_mad<4>(odd, p.v + 1, m);
+    row_mad_c<4>(even, p.v, m, odd[7]);
+}
+
+// a b R^-1 mod p in [0, 2p)
+template <class Params>
+__host__ __device__ __forceinline__ void mul_redc(const uint32_t* a, const uint32_t* b, uint32_t* r) {
+    uint32_t x[8], y[8];
+    row_mul<4>(x, a, b[0]);
+    row_mul<4>(y, a + 1, b[0]);
+    reduce_row<Params>(x, y);
+#pragma unroll
+    for (int i = 1; i < 8; i += 2) {   // the vectors trade places with every limb
+        row_shift_mad(x, y[0], a + 1, b[i]);
+        row_mad_c<4>(y, a, b[i], x[7]);
+        reduce_row<Params>(y, x);
+        if (i + 1 < 8) {
+            row_shift_mad(y, x[0], a + 1, b[i + 1]);
+            row_mad_c<4>(x, a, b[i + 1], y[7]);
+            reduce_row<Params>(x, y);
+        }
+    }
+    merge_odd_even(r, x, y);
+}
+
 template <class Params>
 __device__ __forceinline__ Fp<Params> mul(const Fp<Params>& a, const Fp<Params>& b) {
-    uint32_t t[10];
-#pragma unroll
-    for (int i = 0; i < 10; i++) t[i] = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        uint64_t c = 0;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            uint64_t p = (uint64_t)a.v[j] * b.v[i] + t[j] + c;
-            t[j] = (uint32_t)p;
-            c = p >> 32;
-        }
-        uint64_t s = (uint64_t)t[8] + c;
-        t[8] = (uint32_t)s;
-        t[9] = (uint32_t)(s >> 32);
-        // m = t0 * (-p^-1) mod 2^32 makes t + m p divisible by 2^32
-        uint32_t m = t[0] * Params::N0;
-        c = ((uint64_t)m * Params::P(0) + t[0]) >> 32;
-#pragma unroll
-        for (int j = 1; j < 8; j++) {
-            uint64_t p = (uint64_t)m * Params::P(j) + t[j] + c;
-            t[j - 1] = (uint32_t)p;
-            c = p >> 32;
-        }
-        s = (uint64_t)t[8] + c;
-        t[7] = (uint32_t)s;
-        t[8] = t[9] + (uint32_t)(s >> 32);
-    }
-    reduce_once<Params>(t);
     Fp<Params> r;
-#pragma unroll
-    for (int i = 0; i < 8; i++) r.v[i] = t[i];
+    mul_redc<Params>(a.v, b.v, r.v);
+    reduce_once<Params>(r.v);
     return r;
 }
 
 // Montgomery reduction of a 16-limb t < p R: t R^-1 mod p, left in [0, 2p)
-// in r[0..7] (t is clobbered).  Row i adds m p 2^(32 i), m = t[i] (-p^-1) mod
-// 2^32, which zeroes limb i; the carry out of limb i + 8 rides into the next
-// row.  (t + M p) / R < 2p < 2^255, so no carry is left at the end.
+// in r[0..7].  The low half is reduced as in mul_redc, the high half added at
+// the end: (t + M p) / R < 2p < 2^255, so no carry is left.
 template <class Params>
-__host__ __device__ __forceinline__ void redc_wide(uint32_t* t, uint32_t* r) {
-    uint32_t extra = 0;
+__host__ __device__ __forceinline__ void redc_wide(const uint32_t* t, uint32_t* r) {
+    const Modulus<Params> p;
+    uint32_t x[8], y[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        uint32_t m = t[i] * Params::N0;
-        uint64_t c = ((uint64_t)m * Params::P(0) + t[i]) >> 32;
+    for (int k = 0; k < 8; k++) x[k] = t[k];
+    uint32_t m = x[0] * Params::N0;
+    row_mul<4>(y, p.v + 1, m);
+    row_mad_c<4>(x, p.v, m, y[7]);
 #pragma unroll
-        for (int j = 1; j < 8; j++) {
-            uint64_t p = (uint64_t)m * Params::P(j) + t[i + j] + c;
-            t[i + j] = (uint32_t)p;
-            c = p >> 32;
+    for (int i = 1; i < 8; i += 2) {
+        m = (y[0] + x[1]) * Params::N0;
+        row_shift_mad(x, y[0], p.v + 1, m);
+        row_mad_c<4>(y, p.v, m, x[7]);
+        if (i + 1 < 8) {
+            m = (x[0] + y[1]) * Params::N0;
+            row_shift_mad(y, x[0], p.v + 1, m);
+            row_mad_c<4>(x, p.v, m, y[7]);
         }
-        uint64_t s = (uint64_t)t[i + 8] + c + extra;
-        t[i + 8] = (uint32_t)s;
-        extra = (uint32_t)(s >> 32);
     }
-#pragma unroll
-    for (int k = 0; k < 8; k++) r[k] = t[k + 8];
+    merge_odd_even(r, x, y);
+    add_words<8>(r, r, t + 8);
 }
 
-// a b as a 16-limb integer (schoolbook rows with 64-bit sums; row i writes
-// limb i + 8 fresh, since the rows before it reach limb i + 7 at most)
+// t = e + o 2^32, the even and odd positions of a product below 2^512
+__host__ __device__ __forceinline__ void merge_wide(uint32_t* t, const uint32_t* e, const uint32_t* o) {
+    const uint32_t up[16] = {0, o[0], o[1], o[2], o[3], o[4], o[5], o[6], o[7], o[8], o[9], o[10], o[11], o[12],
+                             o[13], o[14]};
+    add_words<16>(t, e, up);
+}
+
+// a b as a 16-limb integer.  A row reaches at most two limbs that no row
+// before it wrote, so one of its two chains ends in a fresh lane and the other
+// carries into a fresh limb.
 __host__ __device__ __forceinline__ void mul_wide(const uint32_t* a, const uint32_t* b, uint32_t* t) {
+    uint32_t e[16], o[16];
 #pragma unroll
-    for (int k = 0; k < 16; k++) t[k] = 0;
+    for (int k = 8; k < 16; k++) e[k] = o[k] = 0;
+    row_mul<4>(e, a, b[0]);
+    row_mul<4>(o, a + 1, b[0]);
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        uint64_t c = 0;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            uint64_t p = (uint64_t)a[j] * b[i] + t[i + j] + c;
-            t[i + j] = (uint32_t)p;
-            c = p >> 32;
+    for (int i = 1; i < 8; i++) {
+        if (i & 1) {   // a's even words fall on odd positions
+            row_mad_c<4>(o + i - 1, a, b[i], o[i + 7]);
+            row_mad<4>(e + i + 1, a + 1, b[i]);
+        } else {
+            row_mad_c<4>(e + i, a, b[i], e[i + 8]);
+            row_mad<4>(o + i, a + 1, b[i]);
         }
-        t[i + 8] = (uint32_t)c;
     }
+    merge_wide(t, e, o);
+}
+
+// t += sum a_i^2 2^(64 i), nothing carried out of limb 15
+__host__ __device__ __forceinline__ void sqr_diagonal(uint32_t* t, const uint32_t* a) {
+#ifdef __CUDA_ARCH__
+    asm("mad.lo.cc.u32  %0, %16, %16, %0;\n\t"
+        "madc.hi.cc.u32 %1, %16, %16, %1;\n\t"
+        "madc.lo.cc.u32 %2, %17, %17, %2;\n\t"
+        "madc.hi.cc.u32 %3, %17, %17, %3;\n\t"
+        "madc.lo.cc.u32 %4, %18, %18, %4;\n\t"
+        "madc.hi.cc.u32 %5, %18, %18, %5;\n\t"
+        "madc.lo.cc.u32 %6, %19, %19, %6;\n\t"
+        "madc.hi.cc.u32 %7, %19, %19, %7;\n\t"
+        "madc.lo.cc.u32 %8, %20, %20, %8;\n\t"
+        "madc.hi.cc.u32 %9, %20, %20, %9;\n\t"
+        "madc.lo.cc.u32 %10, %21, %21, %10;\n\t"
+        "madc.hi.cc.u32 %11, %21, %21, %11;\n\t"
+        "madc.lo.cc.u32 %12, %22, %22, %12;\n\t"
+        "madc.hi.cc.u32 %13, %22, %22, %13;\n\t"
+        "madc.lo.cc.u32 %14, %23, %23, %14;\n\t"
+        "madc.hi.u32    %15, %23, %23, %15;"
+        : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]),
+          "+r"(t[8]), "+r"(t[9]), "+r"(t[10]), "+r"(t[11]), "+r"(t[12]), "+r"(t[13]), "+r"(t[14]), "+r"(t[15])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]));
+#else
+    uint32_t carry = 0;
+    for (int i = 0; i < 8; i++) {
+        const uint64_t x = (uint64_t)t[2 * i + 1] << 32 | t[2 * i], p = (uint64_t)a[i] * a[i], s = x + p, r = s + carry;
+        carry = (uint32_t)(s < x) + (uint32_t)(r < s);
+        t[2 * i] = (uint32_t)r;
+        t[2 * i + 1] = (uint32_t)(r >> 32);
+    }
+#endif
 }
 
 // a^2 R^-1 mod p, left in [0, 2p) in r[0..7] (separated operand scanning):
-// the 28 cross products a_i a_j (i < j) once, doubled by a one-bit shift, plus
-// the 8 squares a_i^2, then a Montgomery reduction of the 16-limb square.  36
-// limb products and 64 for the reduction against CIOS's 128: the same REDC
-// value (a^2 + M p) / R, M being the unique multiple in [0, R), so the result
-// is identical to mul(a, a).  Host-callable for the unit check of the limbs.
+// the 28 cross products a_i a_j (i < j) once, doubled, plus the 8 squares
+// a_i^2, then a Montgomery reduction of the 16-limb square.  36 limb products
+// and 64 for the reduction against 128: the same REDC value (a^2 + M p) / R, M
+// being the unique multiple in [0, R), so the result is identical to
+// mul(a, a).
 template <class Params>
 __host__ __device__ __forceinline__ void sqr_redc(const uint32_t* a, uint32_t* r) {
-    uint32_t t[16];
+    // a_i a_j at position i + j; o[k] is position k + 1
+    uint32_t e[16], o[16], t[16];
 #pragma unroll
-    for (int k = 0; k < 16; k++) t[k] = 0;
-    // cross products: row i adds a_i a_j (j > i) at limb i + j; t[i + 8] is untouched before row i
-#pragma unroll
-    for (int i = 0; i < 7; i++) {
-        uint64_t c = 0;
-#pragma unroll
-        for (int j = i + 1; j < 8; j++) {
-            uint64_t p = (uint64_t)a[i] * a[j] + t[i + j] + c;
-            t[i + j] = (uint32_t)p;
-            c = p >> 32;
-        }
-        t[i + 8] = (uint32_t)c;
-    }
+    for (int k = 0; k < 16; k++) e[k] = o[k] = 0;
+    row_mul<4>(o, a + 1, a[0]);                // 1, 3, 5, 7
+    row_mul<3>(e + 2, a + 2, a[0]);            // 2, 4, 6
+    row_mad_c<3>(o + 2, a + 2, a[1], o[8]);    // 3, 5, 7
+    row_mad<3>(e + 4, a + 3, a[1]);            // 4, 6, 8
+    row_mad<3>(o + 4, a + 3, a[2]);            // 5, 7, 9
+    row_mad_c<2>(e + 6, a + 4, a[2], e[10]);   // 6, 8
+    row_mad_c<2>(o + 6, a + 4, a[3], o[10]);   // 7, 9
+    row_mad<2>(e + 8, a + 5, a[3]);            // 8, 10
+    row_mad<2>(o + 8, a + 5, a[4]);            // 9, 11
+    row_mad_c<1>(e + 10, a + 6, a[4], e[12]);  // 10
+    row_mad_c<1>(o + 10, a + 6, a[5], o[12]);  // 11
+    row_mad<1>(e + 12, a + 7, a[5]);           // 12
+    row_mad<1>(o + 12, a + 7, a[6]);           // 13
+    merge_wide(t, e, o);
     // double (the cross sum is below 2^511, so the shift loses nothing)
-    t[15] = t[14] >> 31;
 #pragma unroll
-    for (int k = 14; k >= 1; k--) t[k] = (t[k] << 1) | (t[k - 1] >> 31);
+    for (int k = 15; k >= 1; k--) t[k] = (t[k] << 1) | (t[k - 1] >> 31);
     // t[0] is zero: no cross product lands on limb 0
-    // add the squares a_i^2 at limbs 2i, 2i + 1
-    {
-        uint64_t c = 0;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            uint64_t q = (uint64_t)a[i] * a[i];
-            uint64_t s0 = (uint64_t)t[2 * i] + (uint32_t)q + c;
-            t[2 * i] = (uint32_t)s0;
-            uint64_t s1 = (uint64_t)t[2 * i + 1] + (q >> 32) + (s0 >> 32);
-            t[2 * i + 1] = (uint32_t)s1;
-            c = s1 >> 32;
-        }
-    }
+    sqr_diagonal(t, a);
     redc_wide<Params>(t, r);
 }
 
@@ -384,12 +615,19 @@ __device__ __forceinline__ Fp<Params> sqr(const Fp<Params>& a) {
     return r;
 }
 
-// Montgomery -> standard form: a * 1 * R^-1
+// Montgomery -> standard form: a R^-1, the reduction alone
 template <class Params>
 __device__ __forceinline__ Fp<Params> from_mont(const Fp<Params>& a) {
-    Fp<Params> one_raw = Fp<Params>::zero();
-    one_raw.v[0] = 1;
-    return mul(a, one_raw);
+    uint32_t t[16];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        t[i] = a.v[i];
+        t[i + 8] = 0;
+    }
+    Fp<Params> r;
+    redc_wide<Params>(t, r.v);
+    reduce_once<Params>(r.v);
+    return r;
 }
 
 typedef Fp<FrParams> Fr;
@@ -408,43 +646,37 @@ __device__ __forceinline__ Fq2 sub(const Fq2& a, const Fq2& b) { return {sub(a.c
 __device__ __forceinline__ Fq2 neg(const Fq2& a) { return {neg(a.c0), neg(a.c1)}; }
 __device__ __forceinline__ Fq2 dbl(const Fq2& a) { return {dbl(a.c0), dbl(a.c1)}; }
 // (a b - c d) R^-1 mod p, left in [0, 2p), with one Montgomery reduction
-// instead of two: the 512-bit a b + p^2 - c d is positive and below 2 p^2 < p R
-// for inputs below p, and its reduction equals (a b R^-1 - c d R^-1) mod p.
-// c d is subtracted row by row; the borrow out of limb i + 8 rides into the
-// next row, as the carry does in redc_wide (the running value never drops
-// below a b + p^2 - c d > 0).  Params must carry p^2 (P2W).  Host-callable.
+// instead of two: a b + (p - c) d, row by row as in mul_redc with two
+// products a row.  The sum is below 2 p^2, the running value below
+// 3 p 2^32 < 2^288 as before, and the result below 2p.
 template <class Params>
 __host__ __device__ __forceinline__ void mul_sub_redc(const uint32_t* a, const uint32_t* b, const uint32_t* c,
                                                       const uint32_t* d, uint32_t* r) {
-    uint32_t t[16];
-    mul_wide(a, b, t);
-    {
-        uint64_t k = 0;
+    const Modulus<Params> p;
+    uint32_t n[8];   // p - c
+    sub_words<8>(n, p.v, c);
+    uint32_t x[8], y[8];
+    row_mul<4>(x, a, b[0]);
+    row_mul<4>(y, a + 1, b[0]);
+    row_mad<4>(y, n + 1, d[0]);
+    row_mad_c<4>(x, n, d[0], y[7]);
+    reduce_row<Params>(x, y);
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            k += (uint64_t)t[i] + Params::P2W(i);
-            t[i] = (uint32_t)k;
-            k >>= 32;
+    for (int i = 1; i < 8; i += 2) {
+        row_shift_mad(x, y[0], a + 1, b[i]);
+        row_mad_c<4>(y, a, b[i], x[7]);
+        row_mad<4>(x, n + 1, d[i]);
+        row_mad_c<4>(y, n, d[i], x[7]);
+        reduce_row<Params>(y, x);
+        if (i + 1 < 8) {
+            row_shift_mad(y, x[0], a + 1, b[i + 1]);
+            row_mad_c<4>(x, a, b[i + 1], y[7]);
+            row_mad<4>(y, n + 1, d[i + 1]);
+            row_mad_c<4>(x, n, d[i + 1], y[7]);
+            reduce_row<Params>(x, y);
         }
     }
-    int64_t pend = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        uint64_t cy = 0;
-        int64_t br = 0;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            uint64_t pr = (uint64_t)c[j] * d[i] + cy;
-            cy = pr >> 32;
-            int64_t x = (int64_t)t[i + j] - (int64_t)(uint32_t)pr + br;
-            t[i + j] = (uint32_t)x;
-            br = x >> 32;
-        }
-        int64_t x = (int64_t)t[i + 8] - (int64_t)cy + br + pend;
-        t[i + 8] = (uint32_t)x;
-        pend = x >> 32;
-    }
-    redc_wide<Params>(t, r);
+    merge_odd_even(r, x, y);
 }
 
 // a b - c d in Fq with one reduction (mul_sub_redc)
@@ -467,35 +699,18 @@ __device__ __forceinline__ Fq mul_sub(const Fq& a, const Fq& b, const Fq& c, con
 // Inputs below q.  Host-callable for the unit check of the limbs.
 __host__ __device__ __forceinline__ void fq2_mul_redc(const uint32_t* a0, const uint32_t* a1, const uint32_t* b0,
                                                       const uint32_t* b1, uint32_t* r0, uint32_t* r1) {
-    uint32_t t0[16], t1[16], m[16], sa[8], sb[8];
-    {
-        uint64_t ca = 0, cb = 0;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            ca += (uint64_t)a0[i] + a1[i];
-            sa[i] = (uint32_t)ca;
-            ca >>= 32;
-            cb += (uint64_t)b0[i] + b1[i];
-            sb[i] = (uint32_t)cb;
-            cb >>= 32;
-        }
-    }
+    uint32_t t0[16], t1[16], m[16], sa[8], sb[8], q2[16];
+    add_words<8>(sa, a0, a1);
+    add_words<8>(sb, b0, b1);
     mul_wide(a0, b0, t0);
     mul_wide(a1, b1, t1);
     mul_wide(sa, sb, m);
-    // m -= t0 + t1;  t0 += q^2 - t1
-    {
-        int64_t bm = 0, b0w = 0;
+    sub_words<16>(m, m, t0);
+    sub_words<16>(m, m, t1);
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            int64_t dm = (int64_t)m[i] - t0[i] - t1[i] + bm;
-            m[i] = (uint32_t)dm;
-            bm = dm >> 32;   // arithmetic shift: 0, -1 or -2
-            int64_t d0 = (int64_t)t0[i] + FqParams::P2W(i) - t1[i] + b0w;
-            t0[i] = (uint32_t)d0;
-            b0w = d0 >> 32;  // -1, 0 or 1
-        }
-    }
+    for (int i = 0; i < 16; i++) q2[i] = FqParams::P2W(i);
+    add_words<16>(t0, t0, q2);
+    sub_words<16>(t0, t0, t1);
     redc_wide<FqParams>(t0, r0);
     redc_wide<FqParams>(m, r1);
 }

@@ -41,11 +41,6 @@ __device__ __forceinline__ void st_g(uint4* g, size_t i, const Fr& x) {
     g[2 * i + 1] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
 }
 
-// The butterflies, the coset multiply and the join use mul, the CIOS product
-// on 32x32->64-bit multiply-adds (field.cuh), which measured faster than the
-// PTX carry-chain form mul_cc; the table builders below keep mul_cc, so both
-// forms stay under the parity tests.
-
 // One radix-2 stage on a shared-memory tile.  The tile holds elements
 // i = hi*2^(s_lo+k) + mid*2^s_lo + (lo0 + l) at smem slot mid*L + l; stage
 // s = s_lo + j pairs mid values differing in bit j.  The butterfly's
@@ -238,8 +233,8 @@ __global__ void __launch_bounds__(256) k_ntt_mid_multi(const NttJob* __restrict_
 __device__ __forceinline__ Fr fr_pow_u64(Fr b, uint64_t e) {
     Fr acc = Fr::one();
     while (e) {
-        if (e & 1) acc = mul_cc(acc, b);
-        b = mul_cc(b, b);
+        if (e & 1) acc = mul(acc, b);
+        b = mul(b, b);
         e >>= 1;
     }
     return acc;
@@ -250,11 +245,11 @@ __global__ void k_powers(uint4* out, Fr base, Fr scale, uint64_t count, uint32_t
     uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint64_t i0 = t * 16;
     if (i0 >= count) return;
-    Fr p = mul_cc(scale, fr_pow_u64(base, i0));
+    Fr p = mul(scale, fr_pow_u64(base, i0));
     for (uint64_t i = i0; i < i0 + 16 && i < count; i++) {
         size_t dst = bitrev_log ? (size_t)(__brevll(i) >> (64 - bitrev_log)) : (size_t)i;
         st_g(out, dst, p);
-        p = mul_cc(p, base);
+        p = mul(p, base);
     }
 }
 
@@ -265,8 +260,8 @@ __global__ void k_distribute(uint4* a, Fr shift, uint64_t n) {
     if (i0 >= n) return;
     Fr p = fr_pow_u64(shift, i0);
     for (uint64_t i = i0; i < i0 + 16 && i < n; i++) {
-        st_g(a, i, mul_cc(ld_rw(a, i), p));
-        p = mul_cc(p, shift);
+        st_g(a, i, mul(ld_rw(a, i), p));
+        p = mul(p, shift);
     }
 }
 
@@ -284,7 +279,7 @@ __global__ void k_bitrev(uint4* a, uint32_t log_n, uint64_t n) {
 __global__ void k_join(const uint4* a, const uint4* b, const uint4* c, uint4* h, uint64_t n) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    st_g(h, i, sub(mul_cc(ld_rw(a, i), ld_rw(b, i)), ld_rw(c, i)));
+    st_g(h, i, sub(mul(ld_rw(a, i), ld_rw(b, i)), ld_rw(c, i)));
 }
 
 }  // namespace g16d
