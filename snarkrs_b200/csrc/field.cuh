@@ -645,38 +645,45 @@ __device__ __forceinline__ Fq2 add(const Fq2& a, const Fq2& b) { return {add(a.c
 __device__ __forceinline__ Fq2 sub(const Fq2& a, const Fq2& b) { return {sub(a.c0, b.c0), sub(a.c1, b.c1)}; }
 __device__ __forceinline__ Fq2 neg(const Fq2& a) { return {neg(a.c0), neg(a.c1)}; }
 __device__ __forceinline__ Fq2 dbl(const Fq2& a) { return {dbl(a.c0), dbl(a.c1)}; }
-// (a b - c d) R^-1 mod p, left in [0, 2p), with one Montgomery reduction
-// instead of two: a b + (p - c) d, row by row as in mul_redc with two
-// products a row.  The sum is below 2 p^2, the running value below
-// 3 p 2^32 < 2^288 as before, and the result below 2p.
+// (a b + c d) R^-1 mod p, left in [0, 2p), with one Montgomery reduction
+// instead of two, row by row as in mul_redc with two products a row.  Operands
+// up to p: the running value stays below 3 p 2^32 < 2^288 and the result below
+// 2p.
 template <class Params>
-__host__ __device__ __forceinline__ void mul_sub_redc(const uint32_t* a, const uint32_t* b, const uint32_t* c,
+__host__ __device__ __forceinline__ void mul_add_redc(const uint32_t* a, const uint32_t* b, const uint32_t* c,
                                                       const uint32_t* d, uint32_t* r) {
-    const Modulus<Params> p;
-    uint32_t n[8];   // p - c
-    sub_words<8>(n, p.v, c);
     uint32_t x[8], y[8];
     row_mul<4>(x, a, b[0]);
     row_mul<4>(y, a + 1, b[0]);
-    row_mad<4>(y, n + 1, d[0]);
-    row_mad_c<4>(x, n, d[0], y[7]);
+    row_mad<4>(y, c + 1, d[0]);
+    row_mad_c<4>(x, c, d[0], y[7]);
     reduce_row<Params>(x, y);
 #pragma unroll
     for (int i = 1; i < 8; i += 2) {
         row_shift_mad(x, y[0], a + 1, b[i]);
         row_mad_c<4>(y, a, b[i], x[7]);
-        row_mad<4>(x, n + 1, d[i]);
-        row_mad_c<4>(y, n, d[i], x[7]);
+        row_mad<4>(x, c + 1, d[i]);
+        row_mad_c<4>(y, c, d[i], x[7]);
         reduce_row<Params>(y, x);
         if (i + 1 < 8) {
             row_shift_mad(y, x[0], a + 1, b[i + 1]);
             row_mad_c<4>(x, a, b[i + 1], y[7]);
-            row_mad<4>(y, n + 1, d[i + 1]);
-            row_mad_c<4>(x, n, d[i + 1], y[7]);
+            row_mad<4>(y, c + 1, d[i + 1]);
+            row_mad_c<4>(x, c, d[i + 1], y[7]);
             reduce_row<Params>(x, y);
         }
     }
     merge_odd_even(r, x, y);
+}
+
+// (a b - c d) R^-1 mod p, left in [0, 2p): a b + (p - c) d
+template <class Params>
+__host__ __device__ __forceinline__ void mul_sub_redc(const uint32_t* a, const uint32_t* b, const uint32_t* c,
+                                                      const uint32_t* d, uint32_t* r) {
+    const Modulus<Params> p;
+    uint32_t n[8];
+    sub_words<8>(n, p.v, c);
+    mul_add_redc<Params>(a, b, n, d, r);
 }
 
 // a b - c d in Fq with one reduction (mul_sub_redc)

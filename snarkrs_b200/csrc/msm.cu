@@ -2,7 +2,7 @@
 #include "msm.cuh"
 #include <type_traits>
 #include "common.cuh"
-#include "curve.cuh"
+#include "lanes.cuh"
 #include <algorithm>
 #include <cstdlib>
 #include <atomic>
@@ -499,33 +499,23 @@ __device__ __forceinline__ uint32_t n_partials(const uint32_t* offsets, uint32_t
     return hi > lo ? ((hi - 1) / L - lo / L + 1) : 0;
 }
 
-// Block-wide sum of one XYZZ point per thread through shared memory; the
-// result is valid in thread 0.
+// ---- bucket reduction: point operations by groups of lanes (lanes.cuh) ----
+constexpr unsigned LANES_BLOCK = 256;   // threads per block of the kernels below
 template <class F>
-__device__ __forceinline__ Xyzz<F> block_sum(Xyzz<F> acc, uint4* smem) {
-    st_xyzz<F>(smem, threadIdx.x, acc);
-    __syncthreads();
-    for (uint32_t s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-            acc = xyzz_add<F, false>(acc, ld_xyzz<F>(smem, threadIdx.x + s));
-            st_xyzz<F>(smem, threadIdx.x, acc);
-        }
-        __syncthreads();
-    }
-    return acc;
-}
+constexpr uint32_t LANES_GROUPS = LANES_BLOCK / Lanes<F>::N;   // points a block works on at a time
 
 // Fat buckets, stage 1: each of a fat bucket's partials is assigned to one of
 // FAT_JOBS contiguous jobs; a block folds one job into the job's first slot.
 template <class F>
-__global__ void __launch_bounds__(128) k_fat_merge_jobs(uint4* __restrict__ partials,
-                                                        const uint32_t* __restrict__ offsets,
-                                                        const uint32_t* __restrict__ seg_base,
-                                                        const uint32_t* __restrict__ fat_list,
-                                                        const uint32_t* __restrict__ fat_count,
-                                                        const uint32_t* __restrict__ d_L) {
-    extern __shared__ uint4 smem[];
-    const uint32_t L = *d_L;
+__global__ void __launch_bounds__(LANES_BLOCK) k_fat_merge_jobs(uint4* __restrict__ partials,
+                                                                const uint32_t* __restrict__ offsets,
+                                                                const uint32_t* __restrict__ seg_base,
+                                                                const uint32_t* __restrict__ fat_list,
+                                                                const uint32_t* __restrict__ fat_count,
+                                                                const uint32_t* __restrict__ d_L) {
+    constexpr uint32_t G = LANES_GROUPS<F>;
+    __shared__ uint4 smem[LANES_BLOCK * 2];
+    const uint32_t L = *d_L, grp = threadIdx.x / Lanes<F>::N;
     uint32_t items = *fat_count * FAT_JOBS;
     for (uint32_t item = blockIdx.x; item < items; item += gridDim.x) {
         uint32_t g = fat_list[item / FAT_JOBS], j = item % FAT_JOBS;
@@ -533,10 +523,11 @@ __global__ void __launch_bounds__(128) k_fat_merge_jobs(uint4* __restrict__ part
         uint32_t a = j * J;
         if (a >= ns) continue;   // uniform across the block
         uint32_t b = min(a + J, ns), base = seg_base[g];
-        Xyzz<F> acc = Xyzz<F>::identity();
-        for (uint32_t i = a + threadIdx.x; i < b; i += blockDim.x) acc = xyzz_add<F, false>(acc, ld_xyzz<F>(partials, base + i));
-        acc = block_sum(acc, smem);
-        if (threadIdx.x == 0) st_xyzz<F>(partials, base + a, acc);
+        Fq acc = a + grp < b ? ld_lane<F>(partials, base + a + grp) : Fq::zero();
+        for (uint32_t i0 = a + G; i0 < b; i0 += G)
+            acc = lanes_add<F>(acc, i0 + grp < b ? ld_lane<F>(partials, base + i0 + grp) : Fq::zero());
+        acc = block_sum_lanes<F>(acc, smem, G);
+        if (grp == 0) st_lane<F>(partials, base + a, acc);
         __syncthreads();
     }
 }
@@ -544,70 +535,61 @@ __global__ void __launch_bounds__(128) k_fat_merge_jobs(uint4* __restrict__ part
 // Fat buckets, stage 2: fold the (at most FAT_JOBS) job results into the
 // bucket's first partial slot.
 template <class F>
-__global__ void __launch_bounds__(64) k_fat_merge_final(uint4* __restrict__ partials,
-                                                        const uint32_t* __restrict__ offsets,
-                                                        const uint32_t* __restrict__ seg_base,
-                                                        const uint32_t* __restrict__ fat_list,
-                                                        const uint32_t* __restrict__ fat_count,
-                                                        const uint32_t* __restrict__ d_L) {
-    extern __shared__ uint4 smem[];
-    const uint32_t L = *d_L;
+__global__ void __launch_bounds__(LANES_BLOCK) k_fat_merge_final(uint4* __restrict__ partials,
+                                                                 const uint32_t* __restrict__ offsets,
+                                                                 const uint32_t* __restrict__ seg_base,
+                                                                 const uint32_t* __restrict__ fat_list,
+                                                                 const uint32_t* __restrict__ fat_count,
+                                                                 const uint32_t* __restrict__ d_L) {
+    constexpr uint32_t G = LANES_GROUPS<F>;
+    __shared__ uint4 smem[LANES_BLOCK * 2];
+    const uint32_t L = *d_L, grp = threadIdx.x / Lanes<F>::N;
     uint32_t nf = *fat_count;
     for (uint32_t f = blockIdx.x; f < nf; f += gridDim.x) {
         uint32_t g = fat_list[f];
         uint32_t ns = n_partials(offsets, g, L), J = fat_job_len(ns);
         uint32_t base = seg_base[g];
-        uint32_t a = threadIdx.x * J;
-        Xyzz<F> acc = a < ns ? ld_xyzz<F>(partials, base + a) : Xyzz<F>::identity();
-        acc = block_sum(acc, smem);
-        if (threadIdx.x == 0) st_xyzz<F>(partials, base, acc);
+        Fq acc = grp * J < ns ? ld_lane<F>(partials, base + grp * J) : Fq::zero();
+        for (uint32_t t0 = G; t0 < FAT_JOBS; t0 += G) {
+            const uint32_t a = (t0 + grp) * J;
+            acc = lanes_add<F>(acc, a < ns ? ld_lane<F>(partials, base + a) : Fq::zero());
+        }
+        acc = block_sum_lanes<F>(acc, smem, G);
+        if (grp == 0) st_lane<F>(partials, base, acc);
         __syncthreads();
     }
 }
 
-// Whether the bucket-sum and reduction kernels inline the G1 addition's
-// products (G16_REDUCE_INLINE_G1=1) or call them out of line (the default).
-#ifndef G16_REDUCE_INLINE_G1
-#define G16_REDUCE_INLINE_G1 0
-#endif
+// Bucket sums S_g: one group of lanes per bucket folds its few partials (a fat
+// bucket's total already sits in its first slot).  A warp's groups run as many
+// steps as its longest bucket needs.
 template <class F>
-constexpr bool REDUCE_INL = std::is_same<F, g16d::Fq>::value && G16_REDUCE_INLINE_G1;
-// Blocks per SM the bucket-sum and pieces kernels' register budget must allow.
-#ifndef REDUCE_MIN_BLOCKS
-#define REDUCE_MIN_BLOCKS 1
-#endif
-
-// Threads per k_bucket_sums block.
-#ifndef G16_BUCKET_SUMS_BLOCK
-#define G16_BUCKET_SUMS_BLOCK 128
-#endif
-constexpr unsigned BUCKET_SUMS_BLOCK = G16_BUCKET_SUMS_BLOCK;
-
-// Bucket sums S_g: one thread per bucket folds its few partials (a fat
-// bucket's total already sits in its first slot).
-template <class F>
-__global__ void __launch_bounds__(BUCKET_SUMS_BLOCK, REDUCE_MIN_BLOCKS) k_bucket_sums(const uint4* __restrict__ partials,
-                                                     const uint32_t* __restrict__ offsets,
-                                                     const uint32_t* __restrict__ seg_base, uint32_t K,
-                                                     const uint32_t* __restrict__ d_L, uint4* __restrict__ buckets) {
-    uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= K) return;
-    const uint32_t L = *d_L;
-    uint32_t ns = n_partials(offsets, g, L), base = seg_base[g];
-    Xyzz<F> acc = Xyzz<F>::identity();
-    if (ns > FAT_PARTIALS) {
-        acc = ld_xyzz<F>(partials, base);
-    } else {
-        for (uint32_t s = 0; s < ns; s++) acc = xyzz_add<F, REDUCE_INL<F>>(acc, ld_xyzz<F>(partials, base + s));
+__global__ void __launch_bounds__(LANES_BLOCK) k_bucket_sums(const uint4* __restrict__ partials,
+                                                             const uint32_t* __restrict__ offsets,
+                                                             const uint32_t* __restrict__ seg_base, uint32_t K,
+                                                             const uint32_t* __restrict__ d_L,
+                                                             uint4* __restrict__ buckets) {
+    const uint32_t g = (blockIdx.x * LANES_BLOCK + threadIdx.x) / Lanes<F>::N;
+    uint32_t ns = 0, base = 0;
+    if (g < K) {
+        ns = n_partials(offsets, g, *d_L);
+        base = seg_base[g];
+        if (ns > FAT_PARTIALS) ns = 1;
     }
-    st_xyzz<F>(buckets, g, acc);
+    const uint32_t steps = __reduce_max_sync(FULL_WARP, ns);
+    Fq acc = ns ? ld_lane<F>(partials, base) : Fq::zero();
+    for (uint32_t s = 1; s < steps; s++)
+        acc = lanes_add<F>(acc, s < ns ? ld_lane<F>(partials, base + s) : Fq::zero());
+    if (g < K) st_lane<F>(buckets, g, acc);
 }
 
 // Bucket reduction, step 1.  A set's buckets S_0 .. S_{B-1} (S_b holds the
-// points whose digit is b + 1) are cut into pieces of seg buckets; thread t of
-// block j owns piece p = j 2^LB + t and folds it by running sums into
+// points whose digit is b + 1) are cut into pieces of seg buckets; piece
+// p = j 2^LB + t of block j gives
 //   run_p = sum_i S_{p seg + i},   tot_p = sum_i (i + 1) S_{p seg + i},
 // so that the set's sum_b (b + 1) S_b = sum_p tot_p + seg sum_p p run_p.
+// Two groups of lanes share a piece: the first runs run += S_i, the second
+// tot += run one step behind it, so a bucket costs one addition of latency.
 // The weights p are split over their bits instead of being multiplied out (a
 // double-and-add per piece costs more than the piece's running sums): the
 // block halves its 2^LB run values LB times in shared memory, v_t += v_(t+h)
@@ -615,74 +597,71 @@ __global__ void __launch_bounds__(BUCKET_SUMS_BLOCK, REDUCE_MIN_BLOCKS) k_bucket
 // exactly the folded values whose piece index has bit log2(h) set.  Once
 // frozen, each upper half is summed by a tree that runs alongside the later
 // halvings, so G_j = sum over the pieces with bit j set of run_p ends in slot
-// 2^j after LB steps.  The tot values halve into T on the threads [h, 2h),
-// which the run halving leaves idle (with seg = 1, tot = run and T = R).  Each
-// step costs a thread at most one addition: a dependent XYZZ addition takes
-// microseconds on an otherwise idle SM, so the depth is what counts here.
+// 2^j after LB steps.  The second groups halve the tot values into T meanwhile
+// (with seg = 1, tot = run and T = R).  Each step is one addition deep: depth
+// is what counts here, the device has lanes to spare.
 // The block writes T, G_0 .. G_(LB-1) and its run total R (LB + 2 points).
 template <class F, int LB>
-__global__ void __launch_bounds__(1 << LB, REDUCE_MIN_BLOCKS) k_reduce_pieces(const uint4* __restrict__ buckets, uint32_t B,
-                                                           uint32_t seg, uint4* __restrict__ out) {
+__device__ __forceinline__ void reduce_piece_block(const uint4* __restrict__ buckets, size_t g0, bool in_range,
+                                                   uint32_t seg, uint4* __restrict__ out, size_t o0) {
     constexpr uint32_t N = 1u << LB;
-    extern __shared__ uint4 smem[];
-    uint4* s_run = smem;
-    uint4* s_tot = smem + N * 4 * Codec<F>::U4;
-    const uint32_t t = threadIdx.x, set = blockIdx.y;
-    const uint32_t p = blockIdx.x * N + t;
+    __shared__ uint4 s_pts[2][N * Lanes<F>::N * 2];   // run, tot
+    const uint32_t t = threadIdx.x / (2 * Lanes<F>::N);
+    const bool second = (threadIdx.x / Lanes<F>::N) & 1u;
     const bool weighted = seg > 1;   // uniform: tot differs from run
-    // G2: tot waits in shared memory while run is added, so that the two
-    // 64-register points and the addition's operands fit without spilling
-    constexpr bool TOT_SHARED = sizeof(F) > sizeof(g16d::Fq);
-    Xyzz<F> run = Xyzz<F>::identity(), tot = Xyzz<F>::identity();
-    if (TOT_SHARED && weighted) st_xyzz<F>(s_tot, t, tot);
-    if ((size_t)p * seg < B) {
-        const size_t g0 = (size_t)set * B + (size_t)p * seg;
+    const bool reads = in_range && !second;
+    Fq acc = Fq::zero(), next = reads ? ld_lane<F>(buckets, g0 + seg - 1) : Fq::zero();
+    const uint32_t steps = weighted ? seg + 1 : 1;
 #pragma unroll 1
-        for (int i = (int)seg - 1; i >= 0; i--) {
-            run = xyzz_add<F, REDUCE_INL<F>>(run, ld_xyzz<F>(buckets, g0 + i));
-            if (weighted) {
-                if constexpr (TOT_SHARED) st_xyzz<F>(s_tot, t, xyzz_add<F, REDUCE_INL<F>>(ld_xyzz<F>(s_tot, t), run));
-                else tot = xyzz_add<F, REDUCE_INL<F>>(tot, run);
-            }
-        }
+    for (uint32_t j = 0; j < steps; j++) {
+        const Fq o = pick(second, shfl_xor(acc, Lanes<F>::N), next);
+        next = reads && j + 1 < seg ? ld_lane<F>(buckets, g0 + seg - 2 - j) : Fq::zero();
+        acc = lanes_add<F>(acc, o);
     }
-    // run stays equal to slot t of s_run: thread t is the only writer of slot t
-    st_xyzz<F>(s_run, t, run);
-    if (!TOT_SHARED && weighted) st_xyzz<F>(s_tot, t, tot);
+    uint4* mine = s_pts[second];
+    // acc stays equal to this group's slot t: no other group writes it
+    st_lane<F>(mine, t, acc);
     const uint32_t lg = t ? 31 - __clz(t) : 0;   // slot t lies in the upper half [2^lg, 2^(lg+1))
 #pragma unroll 1
     for (uint32_t k = 1; k <= (uint32_t)LB; k++) {
         __syncthreads();
         const uint32_t h = N >> k;
-        // a step reads no slot that another thread writes in the same step:
-        // run halving reads [h, 2h) and writes [0, h); the tot halving on
-        // thread t in [h, 2h) reads t - h and t and writes t - h; the trees
-        // stay at 2h and above
+        // a step reads no slot that another group writes in the same step: the
+        // halvings read [h, 2h) and write [0, h); the trees stay at 2h and above
+        uint32_t src = t;   // t: nothing to add in this step
         if (t < h) {
-            run = xyzz_add<F, REDUCE_INL<F>>(run, ld_xyzz<F>(s_run, t + h));
-            st_xyzz<F>(s_run, t, run);
-        } else if (t < 2 * h) {
-            if (weighted) {
-                tot = xyzz_add<F, REDUCE_INL<F>>(ld_xyzz<F>(s_tot, t - h), ld_xyzz<F>(s_tot, t));
-                st_xyzz<F>(s_tot, t - h, tot);   // at the last step (t = 1) this is T
-            }
-        } else {
+            if (!second || weighted) src = t + h;
+        } else if (t >= 2 * h && !second) {
             // the half [2^lg, 2^(lg+1)) froze at step LB - lg; tree level k - (LB - lg) - 1 now
             const uint32_t hs = 1u << lg, s = 1u << (k - (LB - lg) - 1), o = t - hs;
-            if ((o & (2 * s - 1)) == 0 && o + s < hs) {
-                run = xyzz_add<F, REDUCE_INL<F>>(run, ld_xyzz<F>(s_run, t + s));
-                st_xyzz<F>(s_run, t, run);
-            }
+            if ((o & (2 * s - 1)) == 0 && o + s < hs) src = t + s;
+        }
+        const bool adds = src != t;
+        if (__any_sync(FULL_WARP, adds)) {
+            acc = lanes_add<F>(acc, adds ? ld_lane<F>(mine, src) : Fq::zero());
+            if (adds) st_lane<F>(mine, t, acc);
         }
     }
-    const size_t o0 = ((size_t)set * gridDim.x + blockIdx.x) * (LB + 2);
-    if (t == 0) {
-        if (!weighted) st_xyzz<F>(out, o0, run);
-        st_xyzz<F>(out, o0 + LB + 1, run);
+    if (second) {
+        if (t == 0 && weighted) st_lane<F>(out, o0, acc);   // T
+    } else if (t == 0) {
+        if (!weighted) st_lane<F>(out, o0, acc);
+        st_lane<F>(out, o0 + LB + 1, acc);
     } else if ((t & (t - 1)) == 0) {
-        st_xyzz<F>(out, o0 + 1 + lg, run);   // G_lg
-        if (t == 1 && weighted) st_xyzz<F>(out, o0, tot);
+        st_lane<F>(out, o0 + 1 + lg, acc);   // G_lg
     }
+}
+
+// threads of a reduction block: two groups for each of its 2^LB pieces
+template <class F, int LB>
+constexpr unsigned REDUCE_BLOCK = (2u * Lanes<F>::N) << LB;
+
+template <class F, int LB>
+__global__ void __launch_bounds__(REDUCE_BLOCK<F, LB>) k_reduce_pieces(const uint4* __restrict__ buckets, uint32_t B,
+                                                                       uint32_t seg, uint4* __restrict__ out) {
+    const uint32_t p = (blockIdx.x << LB) + threadIdx.x / (2 * Lanes<F>::N), set = blockIdx.y;
+    reduce_piece_block<F, LB>(buckets, (size_t)set * B + (size_t)p * seg, (size_t)p * seg < B, seg, out,
+                              ((size_t)set * gridDim.x + blockIdx.x) * (LB + 2));
 }
 
 // Bucket reduction, step 2 (when a set has more than a couple of blocks):
@@ -691,19 +670,28 @@ __global__ void __launch_bounds__(1 << LB, REDUCE_MIN_BLOCKS) k_reduce_pieces(co
 // totals R of the blocks whose index has bit i set.  The host then forms
 // T + seg (sum_j 2^j G_j + 2^LB sum_i 2^i Gb_i) by doublings and additions.
 template <class F, int LB>
-__global__ void __launch_bounds__(128) k_reduce_sets(const uint4* __restrict__ in, uint32_t nb,
-                                                     uint4* __restrict__ out) {
-    extern __shared__ uint4 smem[];
+__device__ __forceinline__ void reduce_set_term(const uint4* __restrict__ in, size_t base, uint32_t nb, uint32_t o,
+                                                uint4* __restrict__ out, size_t to) {
+    __shared__ uint4 smem[LANES_BLOCK * 2];
+    const uint32_t grp = threadIdx.x / Lanes<F>::N, groups = blockDim.x / Lanes<F>::N;
+    const bool bits = o > (uint32_t)LB;
+    const uint32_t i = bits ? o - LB - 1 : 0, count = bits ? nb / 2 : nb;
+    auto at = [&](uint32_t x) {   // the x-th point of the term
+        const uint32_t j = bits ? ((x >> i) << (i + 1)) | (1u << i) | (x & ((1u << i) - 1u)) : x;
+        return base + (size_t)j * (LB + 2) + (bits ? LB + 1 : o);
+    };
+    Fq acc = grp < count ? ld_lane<F>(in, at(grp)) : Fq::zero();
+    for (uint32_t x0 = groups; x0 < count; x0 += groups)
+        acc = lanes_add<F>(acc, x0 + grp < count ? ld_lane<F>(in, at(x0 + grp)) : Fq::zero());
+    acc = block_sum_lanes<F>(acc, smem, groups);
+    if (grp == 0) st_lane<F>(out, to, acc);
+}
+
+template <class F, int LB>
+__global__ void __launch_bounds__(LANES_BLOCK) k_reduce_sets(const uint4* __restrict__ in, uint32_t nb,
+                                                             uint4* __restrict__ out) {
     const uint32_t o = blockIdx.x, set = blockIdx.y;
-    const size_t base = (size_t)set * nb * (LB + 2);
-    Xyzz<F> acc = Xyzz<F>::identity();
-    for (uint32_t j = threadIdx.x; j < nb; j += blockDim.x) {
-        if (o <= (uint32_t)LB) acc = xyzz_add<F, false>(acc, ld_xyzz<F>(in, base + (size_t)j * (LB + 2) + o));
-        else if ((j >> (o - LB - 1)) & 1u)
-            acc = xyzz_add<F, false>(acc, ld_xyzz<F>(in, base + (size_t)j * (LB + 2) + LB + 1));
-    }
-    acc = block_sum(acc, smem);
-    if (threadIdx.x == 0) st_xyzz<F>(out, (size_t)set * gridDim.x + o, acc);
+    reduce_set_term<F, LB>(in, (size_t)set * nb * (LB + 2), nb, o, out, (size_t)set * gridDim.x + o);
 }
 
 // ---- batched MSMs: several scalar vectors, many MSMs, one launch per step ----
@@ -854,89 +842,31 @@ struct MsmReduceDev {
 // k_reduce_pieces for many segments: block b works on block b - block_start
 // of the segment that owns it, with that segment's B and seg.
 template <class F, int LB>
-__global__ void __launch_bounds__(1 << LB, REDUCE_MIN_BLOCKS) k_reduce_pieces_multi(const uint4* __restrict__ buckets,
-                                                                 const MsmReduceDev* __restrict__ segs,
-                                                                 uint32_t nsegs, uint4* __restrict__ out) {
-    constexpr uint32_t N = 1u << LB;
-    extern __shared__ uint4 smem[];
-    uint4* s_run = smem;
-    uint4* s_tot = smem + N * 4 * Codec<F>::U4;
+__global__ void __launch_bounds__(REDUCE_BLOCK<F, LB>) k_reduce_pieces_multi(const uint4* __restrict__ buckets,
+                                                                             const MsmReduceDev* __restrict__ segs,
+                                                                             uint32_t nsegs, uint4* __restrict__ out) {
     uint32_t lo = 0, hi = nsegs;
     while (hi - lo > 1) {
         uint32_t mid = (lo + hi) >> 1;
         if (segs[mid].block_start <= blockIdx.x) lo = mid; else hi = mid;
     }
     const MsmReduceDev sd = segs[lo];
-    const uint32_t t = threadIdx.x, jb = blockIdx.x - sd.block_start;
-    const uint32_t p = jb * N + t, seg = sd.seg, B = sd.B;
-    const bool weighted = seg > 1;
-    constexpr bool TOT_SHARED = sizeof(F) > sizeof(g16d::Fq);
-    Xyzz<F> run = Xyzz<F>::identity(), tot = Xyzz<F>::identity();
-    if (TOT_SHARED && weighted) st_xyzz<F>(s_tot, t, tot);
-    if ((size_t)p * seg < B) {
-        const size_t g0 = (size_t)sd.key_start + (size_t)p * seg;
-#pragma unroll 1
-        for (int i = (int)seg - 1; i >= 0; i--) {
-            run = xyzz_add<F, REDUCE_INL<F>>(run, ld_xyzz<F>(buckets, g0 + i));
-            if (weighted) {
-                if constexpr (TOT_SHARED) st_xyzz<F>(s_tot, t, xyzz_add<F, REDUCE_INL<F>>(ld_xyzz<F>(s_tot, t), run));
-                else tot = xyzz_add<F, REDUCE_INL<F>>(tot, run);
-            }
-        }
-    }
-    st_xyzz<F>(s_run, t, run);
-    if (!TOT_SHARED && weighted) st_xyzz<F>(s_tot, t, tot);
-    const uint32_t lg = t ? 31 - __clz(t) : 0;
-#pragma unroll 1
-    for (uint32_t k = 1; k <= (uint32_t)LB; k++) {
-        __syncthreads();
-        const uint32_t h = N >> k;
-        if (t < h) {
-            run = xyzz_add<F, REDUCE_INL<F>>(run, ld_xyzz<F>(s_run, t + h));
-            st_xyzz<F>(s_run, t, run);
-        } else if (t < 2 * h) {
-            if (weighted) {
-                tot = xyzz_add<F, REDUCE_INL<F>>(ld_xyzz<F>(s_tot, t - h), ld_xyzz<F>(s_tot, t));
-                st_xyzz<F>(s_tot, t - h, tot);
-            }
-        } else {
-            const uint32_t hs = 1u << lg, s2 = 1u << (k - (LB - lg) - 1), o = t - hs;
-            if ((o & (2 * s2 - 1)) == 0 && o + s2 < hs) {
-                run = xyzz_add<F, REDUCE_INL<F>>(run, ld_xyzz<F>(s_run, t + s2));
-                st_xyzz<F>(s_run, t, run);
-            }
-        }
-    }
-    const size_t o0 = (size_t)sd.out_block + (size_t)jb * (LB + 2);
-    if (t == 0) {
-        if (!weighted) st_xyzz<F>(out, o0, run);
-        st_xyzz<F>(out, o0 + LB + 1, run);
-    } else if ((t & (t - 1)) == 0) {
-        st_xyzz<F>(out, o0 + 1 + lg, run);
-        if (t == 1 && weighted) st_xyzz<F>(out, o0, tot);
-    }
+    const uint32_t jb = blockIdx.x - sd.block_start, p = (jb << LB) + threadIdx.x / (2 * Lanes<F>::N);
+    reduce_piece_block<F, LB>(buckets, (size_t)sd.key_start + (size_t)p * sd.seg, (size_t)p * sd.seg < sd.B, sd.seg,
+                              out, (size_t)sd.out_block + (size_t)jb * (LB + 2));
 }
 
 // k_reduce_sets for many segments: blockIdx.y picks the segment, blockIdx.x
 // the term (T, G_0 .. G_(LB-1), Gb_0 .. Gb_(hb-1)); terms past the segment's
 // own hb leave at once.
 template <class F, int LB>
-__global__ void __launch_bounds__(128) k_reduce_sets_multi(const uint4* __restrict__ in,
-                                                           const MsmReduceDev* __restrict__ segs,
-                                                           uint4* __restrict__ out) {
-    extern __shared__ uint4 smem[];
+__global__ void __launch_bounds__(LANES_BLOCK) k_reduce_sets_multi(const uint4* __restrict__ in,
+                                                                   const MsmReduceDev* __restrict__ segs,
+                                                                   uint4* __restrict__ out) {
     const MsmReduceDev sd = segs[blockIdx.y];
     const uint32_t o = blockIdx.x;
     if (o >= (uint32_t)LB + 1 + sd.hb) return;   // uniform across the block
-    const size_t base = sd.out_block;
-    Xyzz<F> acc = Xyzz<F>::identity();
-    for (uint32_t j = threadIdx.x; j < sd.nb; j += blockDim.x) {
-        if (o <= (uint32_t)LB) acc = xyzz_add<F, false>(acc, ld_xyzz<F>(in, base + (size_t)j * (LB + 2) + o));
-        else if ((j >> (o - LB - 1)) & 1u)
-            acc = xyzz_add<F, false>(acc, ld_xyzz<F>(in, base + (size_t)j * (LB + 2) + LB + 1));
-    }
-    acc = block_sum(acc, smem);
-    if (threadIdx.x == 0) st_xyzz<F>(out, (size_t)sd.out_set + o, acc);
+    reduce_set_term<F, LB>(in, sd.out_block, sd.nb, o, out, (size_t)sd.out_set + o);
 }
 
 // Window-shifted base table: out[w n + i] = 2^(c w) P_i (affine).  Built once
@@ -1389,21 +1319,12 @@ cudaError_t msm_sort_sets(MsmSort* sorts, const MsmLiveSets& sets, const void* d
     return cudaSuccess;
 }
 
-// The pieces kernels keep two points per thread in shared memory: above 48 KB a
-// block needs the opt-in limit (blocks of 2^8 threads).
-static void reduce_attrs() {
-    static const bool done = [] {
-        const int g1 = 2 * (1 << MSM_REDUCE_LB_G1) * (int)XYZZ_G1_BYTES;
-        const int g2 = 2 * (1 << MSM_REDUCE_LB_G2) * (int)XYZZ_G2_BYTES;
-        cudaFuncSetAttribute(k_reduce_pieces<g16d::Fq, MSM_REDUCE_LB_G1>, cudaFuncAttributeMaxDynamicSharedMemorySize, g1);
-        cudaFuncSetAttribute(k_reduce_pieces_multi<g16d::Fq, MSM_REDUCE_LB_G1>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, g1);
-        cudaFuncSetAttribute(k_reduce_pieces<g16d::Fq2, MSM_REDUCE_LB_G2>, cudaFuncAttributeMaxDynamicSharedMemorySize, g2);
-        cudaFuncSetAttribute(k_reduce_pieces_multi<g16d::Fq2, MSM_REDUCE_LB_G2>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, g2);
-        return true;
-    }();
-    (void)done;
+// threads of a k_reduce_sets block: a group per point of a term (nb a power of
+// two), a warp at least
+template <class F>
+static unsigned reduce_sets_threads(uint32_t nb) {
+    const uint32_t t = nb * Lanes<F>::N;
+    return t < 32 ? 32 : t < LANES_BLOCK ? t : LANES_BLOCK;
 }
 
 template <class F>
@@ -1416,7 +1337,6 @@ static cudaError_t accumulate(const MsmSort& s, MsmAccum& acc, const void* d_bas
     const uint32_t Wr = s.shared ? 1u : (uint32_t)s.W;   // bucket sets to reduce
     constexpr bool G2 = !std::is_same<F, g16d::Fq>::value;
     constexpr int LB = G2 ? MSM_REDUCE_LB_G2 : MSM_REDUCE_LB_G1;   // pieces per reduction block: 2^LB
-    reduce_attrs();
     const MsmReducePlan plan =
         msm_reduce_plan(Wr, s.B, G2, s.reduce_pieces ? s.reduce_pieces : msm_reduce_pieces(s.shared));
     acc.plan = plan;
@@ -1444,32 +1364,29 @@ static cudaError_t accumulate(const MsmSort& s, MsmAccum& acc, const void* d_bas
     G16_CUDA(cudaGetLastError());
     {
         TimedLaunch tl("msm_fat_merge", st);
-        k_fat_merge_jobs<F><<<2 * device_sms(), 128, 128 * xyzz_bytes, st>>>(partials, s.d_offsets, s.d_seg_base,
-                                                                          s.d_fat_list,
-                                                                s.d_total + 2, s.d_total + 3);
+        k_fat_merge_jobs<F><<<2 * device_sms(), LANES_BLOCK, 0, st>>>(partials, s.d_offsets, s.d_seg_base, s.d_fat_list,
+                                                                      s.d_total + 2, s.d_total + 3);
     }
     {
         TimedLaunch tl("msm_fat_merge", st);
-        k_fat_merge_final<F><<<device_sms(), 64, 64 * xyzz_bytes, st>>>(partials, s.d_offsets, s.d_seg_base,
-                                                                        s.d_fat_list,
-                                                               s.d_total + 2, s.d_total + 3);
+        k_fat_merge_final<F><<<device_sms(), LANES_BLOCK, 0, st>>>(partials, s.d_offsets, s.d_seg_base, s.d_fat_list,
+                                                                   s.d_total + 2, s.d_total + 3);
     }
     G16_CUDA(cudaGetLastError());
     {
         TimedLaunch tl("msm_bucket_sums", st);
-        k_bucket_sums<F><<<blocks_for(s.K, BUCKET_SUMS_BLOCK), BUCKET_SUMS_BLOCK, 0, st>>>(partials, s.d_offsets, s.d_seg_base, s.K, s.d_total + 3,
-                                                                (uint4*)acc.d_buckets);
+        k_bucket_sums<F><<<blocks_for(s.K, LANES_GROUPS<F>), LANES_BLOCK, 0, st>>>(
+            partials, s.d_offsets, s.d_seg_base, s.K, s.d_total + 3, (uint4*)acc.d_buckets);
     }
     {
         TimedLaunch tl("msm_reduce", st);
         uint4* blocks = (uint4*)(plan.direct ? acc.d_windows : acc.d_segments);
-        k_reduce_pieces<F, LB><<<dim3(plan.nb, Wr), 1u << LB, 2 * ((size_t)1 << LB) * xyzz_bytes, st>>>(
-            (const uint4*)acc.d_buckets, s.B, plan.seg, blocks);
+        k_reduce_pieces<F, LB><<<dim3(plan.nb, Wr), REDUCE_BLOCK<F, LB>, 0, st>>>((const uint4*)acc.d_buckets, s.B,
+                                                                                plan.seg, blocks);
     }
     if (!plan.direct) {
         TimedLaunch tl("msm_reduce", st);
-        const unsigned threads = plan.nb < 128 ? plan.nb : 128;
-        k_reduce_sets<F, LB><<<dim3(LB + 1 + plan.hb, Wr), threads, threads * xyzz_bytes, st>>>(
+        k_reduce_sets<F, LB><<<dim3(LB + 1 + plan.hb, Wr), reduce_sets_threads<F>(plan.nb), 0, st>>>(
             (const uint4*)acc.d_segments, plan.nb, (uint4*)acc.d_windows);
     }
     G16_CUDA(cudaGetLastError());
@@ -1700,28 +1617,28 @@ static cudaError_t space_accumulate(MsmSpace& sp, cudaStream_t st, size_t xyzz_b
     const uint32_t sms = device_sms();
     {
         TimedLaunch tl("msm_fat_merge", st);
-        k_fat_merge_jobs<F><<<2 * sms, 128, 128 * xyzz_bytes, st>>>(partials, s.d_offsets, s.d_seg_base, s.d_fat_list,
-                                                                    s.d_total + 2, s.d_total + 3);
+        k_fat_merge_jobs<F><<<2 * sms, LANES_BLOCK, 0, st>>>(partials, s.d_offsets, s.d_seg_base, s.d_fat_list,
+                                                            s.d_total + 2, s.d_total + 3);
     }
     {
         TimedLaunch tl("msm_fat_merge", st);
-        k_fat_merge_final<F><<<sms, 64, 64 * xyzz_bytes, st>>>(partials, s.d_offsets, s.d_seg_base, s.d_fat_list,
-                                                              s.d_total + 2, s.d_total + 3);
+        k_fat_merge_final<F><<<sms, LANES_BLOCK, 0, st>>>(partials, s.d_offsets, s.d_seg_base, s.d_fat_list,
+                                                          s.d_total + 2, s.d_total + 3);
     }
     G16_CUDA(cudaGetLastError());
     if (s.K) {
         TimedLaunch tl("msm_bucket_sums", st);
-        k_bucket_sums<F><<<blocks_for(s.K, BUCKET_SUMS_BLOCK), BUCKET_SUMS_BLOCK, 0, st>>>(partials, s.d_offsets, s.d_seg_base, s.K, s.d_total + 3,
-                                                                (uint4*)a.d_buckets);
+        k_bucket_sums<F><<<blocks_for(s.K, LANES_GROUPS<F>), LANES_BLOCK, 0, st>>>(
+            partials, s.d_offsets, s.d_seg_base, s.K, s.d_total + 3, (uint4*)a.d_buckets);
     }
     if (sp.blocks) {
         TimedLaunch tl("msm_reduce", st);
-        k_reduce_pieces_multi<F, LB><<<sp.blocks, 1u << LB, 2 * ((size_t)1 << LB) * xyzz_bytes, st>>>(
+        k_reduce_pieces_multi<F, LB><<<sp.blocks, REDUCE_BLOCK<F, LB>, 0, st>>>(
             (const uint4*)a.d_buckets, (const MsmReduceDev*)sp.d_reduce, nsegs, (uint4*)a.d_segments);
     }
     if (nsegs) {
         TimedLaunch tl("msm_reduce_sets", st);
-        k_reduce_sets_multi<F, LB><<<dim3(LB + 1 + sp.max_hb, nsegs), 128, 128 * xyzz_bytes, st>>>(
+        k_reduce_sets_multi<F, LB><<<dim3(LB + 1 + sp.max_hb, nsegs), LANES_BLOCK, 0, st>>>(
             (const uint4*)a.d_segments, (const MsmReduceDev*)sp.d_reduce, (uint4*)a.d_windows);
     }
     G16_CUDA(cudaGetLastError());
@@ -1729,7 +1646,6 @@ static cudaError_t space_accumulate(MsmSpace& sp, cudaStream_t st, size_t xyzz_b
 }
 
 cudaError_t msm_space_accumulate(MsmSpace& sp, cudaStream_t st) {
-    reduce_attrs();
     if (sp.g2) return space_accumulate<g16d::Fq2, MSM_REDUCE_LB_G2>(sp, st, XYZZ_G2_BYTES, "msm_accumulate_g2");
     return space_accumulate<g16d::Fq, MSM_REDUCE_LB_G1>(sp, st, XYZZ_G1_BYTES, "msm_accumulate_g1");
 }

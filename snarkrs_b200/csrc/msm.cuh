@@ -18,13 +18,14 @@
 //      points into XYZZ partial bucket sums, so a fat bucket (a repeated
 //      witness value) is spread over many threads;
 //   4. fat buckets (more than a few partials, e.g. every scalar equal to 1)
-//      are folded by blocks in two tree stages; then one thread per bucket
-//      sums its partials into S_b;
-//   5. the reduction sum_b (b+1) S_b: threads fold pieces of seg buckets by
+//      are folded by blocks in two tree stages; then one group of lanes per
+//      bucket sums its partials into S_b;
+//   5. the reduction sum_b (b+1) S_b: pieces of seg buckets are folded by
 //      running sums, blocks split the pieces' weights over their bits in
 //      shared memory (msm_reduce_plan), a second kernel sums the blocks' bit
-//      terms per set; no step has a long dependent chain, since a dependent
-//      XYZZ addition costs microseconds of latency;
+//      terms per set; no step has a long dependent chain, and every point
+//      operation is spread over a group of lanes (lanes.cuh), since a
+//      dependent XYZZ addition costs microseconds of latency;
 //   6. host: each set's sum from its bit terms, then Horner over the W
 //      window sums (c doublings between windows).
 // One sort serves every base vector that shares the scalars: the prover
@@ -63,21 +64,20 @@ constexpr uint64_t msm_reduce_pieces(bool shared_windows) {
     return shared_windows ? MSM_REDUCE_PIECES : MSM_REDUCE_PIECES_ALONE;
 }
 
-// Pieces per reduction block, 2^LB: one block of 2^LB threads halves its pieces'
-// run sums LB times.  The pieces kernels hold ~250 registers a thread, so 2^8
-// threads is the largest block an SM takes, and a block of 2^8 fills one SM's
-// register file.  The reduction's chains are latency-bound and run beside the
-// other MSMs' accumulations, whose 512-thread blocks each need a whole SM:
-// 8192 pieces as 32 blocks of 2^8 hold 32 SMs, as 64 blocks of 2^7 (or 128 of
-// 2^6, G2) up to 64 (128).  Measured on the 2^21-constraint prove: 2^8 for both
-// groups 53.55-53.61 proofs/s against 53.04-53.20 with 2^7 (G1) and 2^6 (G2),
-// the batched workload 1179-1221 against 1135-1156, although the reduction's
-// own serialized time grows from 2.95 to 3.54 ms per proof.
+// Pieces per reduction block, 2^LB.  A piece takes two groups of lanes
+// (lanes.cuh), 8 lanes over G1 and 16 over G2, so 2^5 and 2^4 pieces make
+// blocks of 256 threads; at under 128 registers two of them fit an SM.  Small
+// blocks spread the pieces over the SMs, and the blocks' terms are summed in
+// parallel by the second kernel.  Against one thread per piece in blocks of 2^8
+// (about 250 registers): the five reductions of a 1.1M-constraint prove 2.41 ->
+// 1.11 ms, of a 2^15-constraint one 1.39 -> 0.64 ms, of a 500-constraint one
+// 0.77 -> 0.21 ms (serialised); a 64-proof batch's, which fill the device
+// either way, 5.8 -> 4.2 ms.
 #ifndef G16_REDUCE_LB_G1
-#define G16_REDUCE_LB_G1 8
+#define G16_REDUCE_LB_G1 5
 #endif
 #ifndef G16_REDUCE_LB_G2
-#define G16_REDUCE_LB_G2 8
+#define G16_REDUCE_LB_G2 4
 #endif
 constexpr uint32_t MSM_REDUCE_LB_G1 = G16_REDUCE_LB_G1;
 constexpr uint32_t MSM_REDUCE_LB_G2 = G16_REDUCE_LB_G2;
@@ -111,8 +111,7 @@ constexpr MsmReducePlan msm_reduce_plan(uint32_t sets, uint32_t B, bool g2, uint
 // bucket set, its first k_reduce_pieces_multi block, its first block-output
 // point (each block writes plan.block_terms() points) and its first result
 // point (plan.set_terms(), summed on the device).  One piece length for the
-// space: its pieces about fill the SMs' resident reduction threads (two
-// blocks of 2^lb, at most 256 threads, per SM), runs of at most 32 buckets;
+// space: its pieces about fill the SMs (two blocks of 2^lb pieces each), runs of at most 32 buckets;
 // piece_len_override (a power of two up to 32) replaces it, and
 // pieces_target (non-zero) replaces the per-segment target.  Host arithmetic
 // only, so that the kernels' indexing can be checked against it on the CPU.
