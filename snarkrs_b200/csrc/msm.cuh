@@ -23,11 +23,10 @@
 //   5. the reduction sum_b (b+1) S_b: pieces of seg buckets are folded by
 //      running sums, blocks split the pieces' weights over their bits in
 //      shared memory (msm_reduce_plan), a second kernel sums the blocks' bit
-//      terms per set; no step has a long dependent chain, and every point
+//      terms per set, a third forms each set's sum; no step has a long dependent chain, and every point
 //      operation is spread over a group of lanes (lanes.cuh), since a
 //      dependent XYZZ addition costs microseconds of latency;
-//   6. host: each set's sum from its bit terms, then Horner over the W
-//      window sums (c doublings between windows).
+//   6. host: Horner over the W window sums (c doublings between windows).
 // One sort serves every base vector that shares the scalars: the prover
 // sorts the witness once and accumulates A, B1, L (G1) and B2 (G2) from it.
 #pragma once
@@ -46,7 +45,7 @@ namespace g16 {
 // shared memory), nb = 2^hb blocks per set.  Each block leaves lb + 2 points, T, G_0 .. G_(lb-1)
 // and its run total R; with more than two blocks in all, a second kernel sums
 // them per set into lb + 1 + hb points, T, G_0 .. G_(lb-1), Gb_0 .. Gb_(hb-1),
-// and the host forms
+// and the last one forms, one block per set,
 //   set sum = T + seg (sum_j 2^j G_j + 2^lb sum_i 2^i Gb_i).
 // seg grows (up to 32) until the pieces over all sets number at most the
 // target.  Fewer, longer pieces keep the reduction's footprint small where it
@@ -71,8 +70,7 @@ constexpr uint64_t msm_reduce_pieces(bool shared_windows) {
 // parallel by the second kernel.  Against one thread per piece in blocks of 2^8
 // (about 250 registers): the five reductions of a 1.1M-constraint prove 2.41 ->
 // 1.11 ms, of a 2^15-constraint one 1.39 -> 0.64 ms, of a 500-constraint one
-// 0.77 -> 0.21 ms (serialised); a 64-proof batch's, which fill the device
-// either way, 5.8 -> 4.2 ms.
+// 0.77 -> 0.21 ms (serialised).
 #ifndef G16_REDUCE_LB_G1
 #define G16_REDUCE_LB_G1 5
 #endif
@@ -84,7 +82,7 @@ constexpr uint32_t MSM_REDUCE_LB_G2 = G16_REDUCE_LB_G2;
 
 struct MsmReducePlan {
     uint32_t sets = 0, B = 0, seg = 1, lb = MSM_REDUCE_LB_G1, nb = 1, hb = 0;
-    bool direct = true;   // the host reads the blocks' own points
+    bool direct = true;   // the last kernel reads the blocks' own points
     constexpr uint32_t block_terms() const { return lb + 2; }
     constexpr uint32_t set_terms() const { return direct ? nb * (lb + 2) : lb + 1 + hb; }
     constexpr size_t block_points() const { return (size_t)sets * nb * (lb + 2); }
@@ -183,11 +181,12 @@ struct MsmAccum {
     void* d_partials = nullptr;    size_t cap_partials = 0;   // bytes
     void* d_buckets = nullptr;     size_t cap_buckets = 0;    // bytes, one XYZZ sum per bucket
     void* d_segments = nullptr;    size_t cap_segments = 0;   // bytes, the reduction blocks' points
-    void* d_windows = nullptr;     size_t cap_windows = 0;    // bytes
+    void* d_terms = nullptr;       size_t cap_terms = 0;      // bytes, the sets' terms
+    void* d_windows = nullptr;     size_t cap_windows = 0;    // bytes, one XYZZ sum per bucket set
     unsigned long long* d_work = nullptr;                      // mixed additions performed
-    MsmReducePlan plan;                                        // shape of d_windows
+    MsmReducePlan plan;
     bool fixed = false;                                        // views, as MsmSort::fixed
-    size_t result_bytes(size_t xyzz_bytes) const { return plan.result_points() * xyzz_bytes; }
+    size_t result_bytes(size_t xyzz_bytes) const { return (size_t)plan.sets * xyzz_bytes; }
     void release();
 };
 
@@ -253,18 +252,17 @@ cudaError_t msm_accumulate_g1(const MsmSort& s, MsmAccum& acc, const void* d_bas
 cudaError_t msm_accumulate_g2(const MsmSort& s, MsmAccum& acc, const void* d_bases, uint32_t base_offset,
                               uint32_t n_bases, cudaStream_t st);
 
-// Host side: the reduction's points (acc.d_windows as copied back, laid out by
-// plan) -> each set's sum -> Horner over the sets with c doublings between
-// them -> Jacobian.
-G1J msm_combine_g1(const uint8_t* result_xyzz, const MsmReducePlan& plan, int c);
-G2J msm_combine_g2(const uint8_t* result_xyzz, const MsmReducePlan& plan, int c);
+// Host side: the sets' sums (acc.d_windows as copied back, plan.sets points)
+// -> Horner over the sets with c doublings between them -> Jacobian.
+G1J msm_combine_g1(const uint8_t* sums_xyzz, const MsmReducePlan& plan, int c);
+G2J msm_combine_g2(const uint8_t* sums_xyzz, const MsmReducePlan& plan, int c);
 
 constexpr size_t XYZZ_G1_BYTES = 128;
 constexpr size_t XYZZ_G2_BYTES = 256;
 
-// The prover reads each of its five MSM results (the reduction's points) back
-// into a pinned host slot of this many bytes: one bucket set with window tables;
-// with a compact key one set per window, W (lb + 1 + hb) points.
+// The prover reads each of its five MSM results (a sum per bucket set) back into
+// a pinned host slot of this many bytes: one bucket set with window tables, one
+// per window with a compact key.
 constexpr size_t MSM_RESULT_SLOT_BYTES = 32 * 256;
 constexpr size_t MSM_RESULT_SLOT_COMPACT_BYTES = 128 * 1024;
 
@@ -300,10 +298,10 @@ struct MsmSpace {
     uint32_t K = 0;                  // buckets over all segments
     uint32_t blocks = 0;             // reduction blocks over all segments
     uint32_t max_hb = 0;
-    uint32_t result_points = 0;      // points of acc.d_windows the host reads
+    uint32_t result_points = 0;      // points of acc.d_windows the host reads, one per segment
     size_t max_entries = 0;
     MsmSort sort;                    // sort buffers over the whole space
-    MsmAccum acc;                    // partials, bucket sums, blocks' points (d_segments), results (d_windows)
+    MsmAccum acc;                    // partials, bucket sums, blocks' points (d_segments), terms (d_terms), results (d_windows)
     void* d_segdev = nullptr;        // accumulate descriptors
     void* d_reduce = nullptr;        // reduction descriptors
     size_t cap_segdev = 0, cap_reduce = 0;

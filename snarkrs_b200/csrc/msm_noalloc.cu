@@ -75,8 +75,10 @@ constexpr size_t BUCKETS_BYTES = g16::XYZZ_G1_BYTES * NOALLOC_K;
 constexpr size_t OFF_SEGMENTS = align256(OFF_BUCKETS + BUCKETS_BYTES);
 constexpr size_t SEGMENTS_BYTES = g16::XYZZ_G1_BYTES * NOALLOC_PLAN.block_points();
 constexpr size_t OFF_WINDOWS = align256(OFF_SEGMENTS + SEGMENTS_BYTES);
-constexpr size_t WINDOWS_BYTES = g16::XYZZ_G1_BYTES * NOALLOC_PLAN.result_points();
-constexpr size_t OFF_WORK = align256(OFF_WINDOWS + WINDOWS_BYTES);
+constexpr size_t WINDOWS_BYTES = g16::XYZZ_G1_BYTES * NOALLOC_PLAN.sets;
+constexpr size_t OFF_TERMS = align256(OFF_WINDOWS + WINDOWS_BYTES);
+constexpr size_t TERMS_BYTES = g16::XYZZ_G1_BYTES * NOALLOC_PLAN.result_points();
+constexpr size_t OFF_WORK = align256(OFF_TERMS + TERMS_BYTES);
 constexpr size_t NOALLOC_SCRATCH_BYTES = align256(OFF_WORK + 8);
 
 // The scratch itself.  In host code this name is only a stand-in for the
@@ -174,6 +176,8 @@ extern "C" int g16_msm_g1_device_noalloc(int device, const void* d_bases, const 
     acc.cap_buckets = BUCKETS_BYTES;
     acc.d_segments = base + OFF_SEGMENTS;
     acc.cap_segments = SEGMENTS_BYTES;
+    acc.d_terms = base + OFF_TERMS;
+    acc.cap_terms = TERMS_BYTES;
     acc.d_windows = base + OFF_WINDOWS;
     acc.cap_windows = WINDOWS_BYTES;
     acc.d_work = (unsigned long long*)(base + OFF_WORK);
