@@ -170,7 +170,8 @@ uint64_t plan_estimate(g16_circuit* const* cs, size_t count) {
         b += (Kw * 2 + c->rows[1] * Ww / 16) * XYZZ_G2_BYTES;
         b += (Kh * 2 + eh / 16) * XYZZ_G1_BYTES;
     }
-    return b + (8ull << 20);
+    // the spaces' smallest chunk counts (msm_max_chunks) past the sixteenths above
+    return b + (8ull << 20) + MSM_SPREAD_THREADS * (2 * XYZZ_G1_BYTES + XYZZ_G2_BYTES);
 }
 
 // device buffer that only grows, reallocated in stream order on st (the engine

@@ -12,6 +12,7 @@ namespace g16d {
 
 using g16::MSM_DEAD;
 using g16::MSM_MAX_SETS;
+using g16::MSM_SPREAD_THREADS;
 using g16::MSM_MAX_TARGETS;
 
 // Bits [off, off + width) of a 256-bit little-endian scalar held in shared
@@ -39,29 +40,63 @@ __device__ __forceinline__ int signed_digit(const uint32_t* s, int w, int c) {
 
 constexpr uint32_t NO_KEY = 0xffffffffu;
 
-// kw: key stride per window (B when every window has its own buckets, 0 when
-// all windows share one bucket set over window-shifted bases)
-// sink: the key of a zero digit (NO_KEY: not sorted; the constant-work sink bucket otherwise)
-__global__ void __launch_bounds__(256) k_digits_count(const uint4* __restrict__ scalars, int mont, uint32_t n, int c,
-                                                      int W, uint32_t kw, uint32_t sink, uint4* __restrict__ scalars_std,
-                                                      uint32_t* __restrict__ counts) {
-    __shared__ uint32_t sh[256 * 9];
-    uint32_t i = blockIdx.x * 256 + threadIdx.x;
-    bool valid = i < n;
+// Scalar i into a shared-memory row of 8 words (zeros when not valid),
+// converted to standard form when mont is set, with a copy to std_out if given.
+__device__ __forceinline__ void stage_scalar(const uint4* __restrict__ scalars, int mont, uint32_t i, bool valid,
+                                             uint4* __restrict__ std_out, uint32_t* row) {
     Fr s = Fr::zero();
     if (valid) {
         uint4 a = __ldg(scalars + 2 * (size_t)i), b = __ldg(scalars + 2 * (size_t)i + 1);
         s.v[0] = a.x; s.v[1] = a.y; s.v[2] = a.z; s.v[3] = a.w;
         s.v[4] = b.x; s.v[5] = b.y; s.v[6] = b.z; s.v[7] = b.w;
         if (mont) s = from_mont(s);
-        scalars_std[2 * (size_t)i] = make_uint4(s.v[0], s.v[1], s.v[2], s.v[3]);
-        scalars_std[2 * (size_t)i + 1] = make_uint4(s.v[4], s.v[5], s.v[6], s.v[7]);
+        if (std_out) {
+            std_out[2 * (size_t)i] = make_uint4(s.v[0], s.v[1], s.v[2], s.v[3]);
+            std_out[2 * (size_t)i + 1] = make_uint4(s.v[4], s.v[5], s.v[6], s.v[7]);
+        }
     }
-    uint32_t* row = sh + threadIdx.x * 9;
 #pragma unroll
     for (int j = 0; j < 8; j++) row[j] = s.v[j];
+}
+
+// A block of 256 threads takes 256 / WPG scalars: WPG warps share 32 scalars
+// and split their windows.  One warp per 32 scalars (WPG = 1) keeps every lane
+// busy in the conversion; below DIGITS_SPLIT scalars its blocks leave most of
+// the SMs empty and the serial loop over the windows is what is waited for, so
+// eight warps split it (1000 scalars of 23 windows: digits 19 -> 7 us, scatter
+// 26 -> 9 us).
+constexpr uint32_t DIGITS_SPLIT = 1u << 18;
+
+template <int WPG>
+struct DigitsPlace {
+    static constexpr uint32_t SCALARS = 256 / WPG;   // per block
+    uint32_t slot;    // this thread's scalar in the block
+    uint32_t i;       // and in the vector
+    int w0;           // its warp's first window; the next ones follow in steps of WPG
+    __device__ __forceinline__ DigitsPlace() {
+        const uint32_t wid = threadIdx.x >> 5;
+        slot = (wid / WPG) * 32 + (threadIdx.x & 31);
+        i = blockIdx.x * SCALARS + slot;
+        w0 = (int)(wid % WPG);
+    }
+};
+
+// kw: key stride per window (B when every window has its own buckets, 0 when
+// all windows share one bucket set over window-shifted bases)
+// sink: the key of a zero digit (NO_KEY: not sorted; the constant-work sink bucket otherwise)
+template <int WPG>
+__global__ void __launch_bounds__(256) k_digits_count(const uint4* __restrict__ scalars, int mont, uint32_t n, int c,
+                                                      int W, uint32_t kw, uint32_t sink, uint4* __restrict__ scalars_std,
+                                                      uint32_t* __restrict__ counts) {
+    __shared__ uint32_t sh[DigitsPlace<WPG>::SCALARS * 9];
+    const DigitsPlace<WPG> at;
+    const uint32_t i = at.i;
+    bool valid = i < n;
+    uint32_t* row = sh + at.slot * 9;
+    if (at.w0 == 0) stage_scalar(scalars, mont, i, valid, scalars_std, row);
+    if (WPG > 1) __syncthreads();
     unsigned lane = threadIdx.x & 31;
-    for (int w = 0; w < W; w++) {
+    for (int w = at.w0; w < W; w += WPG) {
         int d = signed_digit(row, w, c);
         uint32_t key = !valid ? NO_KEY : d != 0 ? (uint32_t)w * kw + (uint32_t)(d < 0 ? -d : d) - 1u : sink;
         unsigned mask = __match_any_sync(0xffffffffu, key);
@@ -71,24 +106,20 @@ __global__ void __launch_bounds__(256) k_digits_count(const uint4* __restrict__ 
 
 // ew: entry-index stride per window (0, or n for window-shifted bases: entry
 // w*n + i names base 2^(c w) P_i)
+template <int WPG>
 __global__ void __launch_bounds__(256) k_scatter(const uint4* __restrict__ scalars_std, uint32_t n, int c, int W,
                                                  uint32_t kw, uint32_t ew, uint32_t sink, uint32_t* __restrict__ cursor,
                                                  uint32_t* __restrict__ entries) {
-    __shared__ uint32_t sh[256 * 9];
-    uint32_t i = blockIdx.x * 256 + threadIdx.x;
+    __shared__ uint32_t sh[DigitsPlace<WPG>::SCALARS * 9];
+    const DigitsPlace<WPG> at;
+    const uint32_t i = at.i;
     bool valid = i < n;
-    uint32_t* row = sh + threadIdx.x * 9;
-    if (valid) {
-        uint4 a = scalars_std[2 * (size_t)i], b = scalars_std[2 * (size_t)i + 1];
-        row[0] = a.x; row[1] = a.y; row[2] = a.z; row[3] = a.w;
-        row[4] = b.x; row[5] = b.y; row[6] = b.z; row[7] = b.w;
-    } else {
-#pragma unroll
-        for (int j = 0; j < 8; j++) row[j] = 0;
-    }
+    uint32_t* row = sh + at.slot * 9;
+    if (at.w0 == 0) stage_scalar(scalars_std, 0, i, valid, nullptr, row);
+    if (WPG > 1) __syncthreads();
     unsigned lane = threadIdx.x & 31;
     unsigned lt = (1u << lane) - 1u;
-    for (int w = 0; w < W; w++) {
+    for (int w = at.w0; w < W; w += WPG) {
         int d = signed_digit(row, w, c);
         uint32_t key = !valid ? NO_KEY : d != 0 ? (uint32_t)w * kw + (uint32_t)(d < 0 ? -d : d) - 1u : sink;
         unsigned mask = __match_any_sync(0xffffffffu, key);
@@ -118,29 +149,22 @@ struct LiveSetArgs {
     uint32_t key_stride;           // bucket offset per window: 0 (one shared set), or B
 };
 
+template <int WPG>
 __global__ void __launch_bounds__(256) k_digits_count_sets(const uint4* __restrict__ scalars, int mont, uint32_t n,
                                                            int c, int W, uint32_t sink, int nsets, LiveSetArgs a,
                                                            uint4* __restrict__ scalars_std) {
-    __shared__ uint32_t sh[256 * 9];
-    uint32_t i = blockIdx.x * 256 + threadIdx.x;
+    __shared__ uint32_t sh[DigitsPlace<WPG>::SCALARS * 9];
+    const DigitsPlace<WPG> at;
+    const uint32_t i = at.i;
     bool valid = i < n;
-    Fr s = Fr::zero();
     bool live[MSM_MAX_SETS];
 #pragma unroll
     for (int j = 0; j < MSM_MAX_SETS; j++) live[j] = valid && j < nsets && __ldg(a.rank[j] + i) != MSM_DEAD;
-    if (valid) {
-        uint4 x = __ldg(scalars + 2 * (size_t)i), y = __ldg(scalars + 2 * (size_t)i + 1);
-        s.v[0] = x.x; s.v[1] = x.y; s.v[2] = x.z; s.v[3] = x.w;
-        s.v[4] = y.x; s.v[5] = y.y; s.v[6] = y.z; s.v[7] = y.w;
-        if (mont) s = from_mont(s);
-        scalars_std[2 * (size_t)i] = make_uint4(s.v[0], s.v[1], s.v[2], s.v[3]);
-        scalars_std[2 * (size_t)i + 1] = make_uint4(s.v[4], s.v[5], s.v[6], s.v[7]);
-    }
-    uint32_t* row = sh + threadIdx.x * 9;
-#pragma unroll
-    for (int j = 0; j < 8; j++) row[j] = s.v[j];
+    uint32_t* row = sh + at.slot * 9;
+    if (at.w0 == 0) stage_scalar(scalars, mont, i, valid, scalars_std, row);
+    if (WPG > 1) __syncthreads();
     unsigned lane = threadIdx.x & 31;
-    for (int w = 0; w < W; w++) {
+    for (int w = at.w0; w < W; w += WPG) {
         int d = signed_digit(row, w, c);
         uint32_t key = d != 0 ? (uint32_t)w * a.key_stride + (uint32_t)(d < 0 ? -d : d) - 1u : sink;
 #pragma unroll
@@ -153,26 +177,22 @@ __global__ void __launch_bounds__(256) k_digits_count_sets(const uint4* __restri
     }
 }
 
+template <int WPG>
 __global__ void __launch_bounds__(256) k_scatter_sets(const uint4* __restrict__ scalars_std, uint32_t n, int c, int W,
                                                       uint32_t sink, int nsets, LiveSetArgs a) {
-    __shared__ uint32_t sh[256 * 9];
-    uint32_t i = blockIdx.x * 256 + threadIdx.x;
+    __shared__ uint32_t sh[DigitsPlace<WPG>::SCALARS * 9];
+    const DigitsPlace<WPG> at;
+    const uint32_t i = at.i;
     bool valid = i < n;
     uint32_t rank[MSM_MAX_SETS];
 #pragma unroll
     for (int j = 0; j < MSM_MAX_SETS; j++) rank[j] = valid && j < nsets ? __ldg(a.rank[j] + i) : MSM_DEAD;
-    uint32_t* row = sh + threadIdx.x * 9;
-    if (valid) {
-        uint4 x = scalars_std[2 * (size_t)i], y = scalars_std[2 * (size_t)i + 1];
-        row[0] = x.x; row[1] = x.y; row[2] = x.z; row[3] = x.w;
-        row[4] = y.x; row[5] = y.y; row[6] = y.z; row[7] = y.w;
-    } else {
-#pragma unroll
-        for (int j = 0; j < 8; j++) row[j] = 0;
-    }
+    uint32_t* row = sh + at.slot * 9;
+    if (at.w0 == 0) stage_scalar(scalars_std, 0, i, valid, nullptr, row);
+    if (WPG > 1) __syncthreads();
     unsigned lane = threadIdx.x & 31;
     unsigned lt = (1u << lane) - 1u;
-    for (int w = 0; w < W; w++) {
+    for (int w = at.w0; w < W; w += WPG) {
         int d = signed_digit(row, w, c);
         uint32_t key = d != 0 ? (uint32_t)w * a.key_stride + (uint32_t)(d < 0 ? -d : d) - 1u : sink;
         const uint32_t sign = d < 0 ? 0x80000000u : 0u;
@@ -190,7 +210,7 @@ __global__ void __launch_bounds__(256) k_scatter_sets(const uint4* __restrict__ 
     }
 }
 
-// ---- exclusive scan (three kernels) ----
+// ---- exclusive scans ----
 __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* warp_tot, uint32_t& total) {
     unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t x = v;
@@ -216,53 +236,6 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* warp_t
     total = warp_tot[nw - 1];
     __syncthreads();
     return before + x - v;
-}
-
-// 1024 elements per block of 256 threads (4 consecutive each)
-__global__ void __launch_bounds__(256) k_scan_blocks(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
-                                                     uint32_t len, uint32_t* __restrict__ block_sums) {
-    __shared__ uint32_t wt[32];
-    size_t base = (size_t)blockIdx.x * 1024 + threadIdx.x * 4;
-    uint32_t v[4], s = 0;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        v[j] = base + j < len ? in[base + j] : 0;
-        s += v[j];
-    }
-    uint32_t total;
-    uint32_t pre = block_excl_scan(s, wt, total);
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        if (base + j < len) out[base + j] = pre;
-        pre += v[j];
-    }
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
-}
-
-// one block of 1024 threads scans nb block sums in place; writes the grand total
-__global__ void __launch_bounds__(1024) k_scan_top(uint32_t* __restrict__ sums, uint32_t nb,
-                                                   uint32_t* __restrict__ total_out) {
-    __shared__ uint32_t wt[32];
-    uint32_t per = (nb + 1023) / 1024;
-    uint32_t lo = threadIdx.x * per, hi = min(lo + per, nb);
-    uint32_t s = 0;
-    for (uint32_t j = lo; j < hi; j++) s += sums[j];
-    uint32_t total;
-    uint32_t pre = block_excl_scan(s, wt, total);
-    for (uint32_t j = lo; j < hi; j++) {
-        uint32_t x = sums[j];
-        sums[j] = pre;
-        pre += x;
-    }
-    if (threadIdx.x == 0) *total_out = total;
-}
-
-__global__ void __launch_bounds__(256) k_scan_add(uint32_t* __restrict__ out, uint32_t len,
-                                                  const uint32_t* __restrict__ sums,
-                                                  const uint32_t* __restrict__ total) {
-    size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
-    if (i < len) out[i] += sums[i / 1024];
-    if (i == 0) out[len] = *total;
 }
 
 // Partial sums per bucket (one per chunk the bucket touches).  Buckets with
@@ -307,25 +280,137 @@ __device__ __forceinline__ uint32_t chunk_len(uint32_t M, uint32_t K, uint32_t L
     return L;
 }
 
-// partials per bucket for the Ks sorted buckets; only the K real ones can be
-// fat (the constant-work sink bucket K is accumulated but never reduced).
-// Also stores the chunk length L in total[3] for the kernels that follow.
-__global__ void k_nseg(const uint32_t* __restrict__ offsets, uint32_t Ks, uint32_t K, uint32_t L_min, uint32_t wave,
-                       uint32_t* __restrict__ nseg, uint32_t* __restrict__ fat_list, uint32_t* __restrict__ fat_count,
-                       uint32_t* __restrict__ total) {
-    uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t L = chunk_len(total[0], K, L_min, wave);
-    if (g == 0) total[3] = L;
-    if (g >= Ks) return;
-    uint32_t lo = offsets[g], hi = offsets[g + 1];
-    uint32_t ns = hi > lo ? ((hi - 1) / L - lo / L + 1) : 0;
-    nseg[g] = ns;
-    if (g < K && ns > FAT_PARTIALS) fat_list[atomicAdd(fat_count, 1u)] = g;
+// Smallest chunk for M entries: down to `floor` (4) entries a thread when 16
+// would leave SMs empty.  A chunk's additions run one after another while its
+// bucket's partial sums cost the bucket-sum step one (dearer) addition each, so
+// the chunks stop shrinking once every SM has its 512 threads.  The four G1
+// accumulates of a 500-constraint prove 0.73 -> 0.12 ms, of a 2^15-constraint
+// one 0.83 -> 0.29 ms, of 1000 uniform points 0.20 -> 0.03 ms.
+__device__ __forceinline__ uint32_t min_chunk(uint32_t M, uint32_t floor) {
+    const uint32_t spread = (M + MSM_SPREAD_THREADS - 1) / MSM_SPREAD_THREADS;
+    const uint32_t L = spread < 16 ? spread : 16;
+    return L > floor ? L : floor;
 }
 
-__global__ void k_copy_u32(uint32_t* dst, const uint32_t* src, uint32_t n) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = src[i];
+// ---- from bucket counts to the accumulate's plan, for up to MSM_MAX_SETS sorts a launch ----
+// Three kernels, blockIdx.y picking the sort, 1024 buckets per block: block sums
+// of the counts; offsets (and the scatter's cursors), the chunk length L, each
+// bucket's partial-sum count and the fat list; the partial sums' bases.  A
+// block adds up the block sums before its own itself (at most a few thousand
+// words from L2) instead of waiting for a kernel that scans them: three
+// launches where scanning twice, copying and counting took eight a sort (a
+// prove's four sorts 32 launches and 0.21 ms serialised, now 6 and 0.05 ms).
+struct SortPlanArgs {
+    uint32_t* counts;     // in: entries per bucket; out: partial sums per bucket
+    uint32_t* offsets;    // Ks + 1
+    uint32_t* cursor;
+    uint32_t* seg_base;   // Ks + 1
+    uint32_t* fat_list;
+    uint32_t* sums;       // block sums of the counts, then those of the partial sums
+    uint32_t* total;      // [0] M, [1] partial sums, [2] fat buckets, [3] L
+    uint32_t Ks, K;       // sorted and real buckets (the constant-work sink is sorted, never reduced)
+    uint32_t L_floor;
+};
+struct SortPlanSets {
+    SortPlanArgs s[MSM_MAX_SETS];
+    uint32_t wave;
+};
+constexpr uint32_t PLAN_BLOCK = 1024;   // buckets per block of 256 threads
+
+// sums[0 .. b) and sums[0 .. nb), by the whole block
+__device__ __forceinline__ uint32_t sums_before(const uint32_t* sums, uint32_t b, uint32_t nb, uint32_t* warp_tot,
+                                                uint32_t& all) {
+    uint32_t before = 0, every = 0;
+    for (uint32_t j = threadIdx.x; j < nb; j += blockDim.x) {
+        const uint32_t x = sums[j];
+        every += x;
+        before += j < b ? x : 0;
+    }
+    uint32_t total;
+    block_excl_scan(every, warp_tot, total);
+    all = total;
+    block_excl_scan(before, warp_tot, total);
+    return total;
+}
+
+__global__ void __launch_bounds__(256) k_plan_sums(SortPlanSets a) {
+    const SortPlanArgs& s = a.s[blockIdx.y];
+    const size_t base = (size_t)blockIdx.x * PLAN_BLOCK + threadIdx.x * 4;
+    if (blockIdx.x && (size_t)blockIdx.x * PLAN_BLOCK >= s.Ks) return;   // uniform across the block
+    __shared__ uint32_t wt[32];
+    uint32_t v = 0, total;
+#pragma unroll
+    for (int j = 0; j < 4; j++) v += base + j < s.Ks ? s.counts[base + j] : 0;
+    block_excl_scan(v, wt, total);
+    if (threadIdx.x == 0) {
+        s.sums[blockIdx.x] = total;
+        if (blockIdx.x == 0) s.total[2] = 0;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_plan_offsets(SortPlanSets a) {
+    const SortPlanArgs& s = a.s[blockIdx.y];
+    const size_t base = (size_t)blockIdx.x * PLAN_BLOCK + threadIdx.x * 4;
+    if (blockIdx.x && (size_t)blockIdx.x * PLAN_BLOCK >= s.Ks) return;   // uniform across the block
+    __shared__ uint32_t wt[32];
+    const uint32_t nb = (s.Ks + PLAN_BLOCK - 1) / PLAN_BLOCK;
+    uint32_t M, total, v[4], sum = 0;
+    const uint32_t before = sums_before(s.sums, blockIdx.x, nb, wt, M);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        v[j] = base + j < s.Ks ? s.counts[base + j] : 0;
+        sum += v[j];
+    }
+    uint32_t off = before + block_excl_scan(sum, wt, total);
+    const uint32_t L = chunk_len(M, s.K, min_chunk(M, s.L_floor), a.wave);
+    uint32_t segs = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const size_t g = base + j;
+        if (g >= s.Ks) break;
+        s.offsets[g] = off;
+        s.cursor[g] = off;
+        const uint32_t hi = off + v[j], ns = v[j] ? ((hi - 1) / L - off / L + 1) : 0;
+        s.counts[g] = ns;
+        if (g < s.K && ns > FAT_PARTIALS) s.fat_list[atomicAdd(s.total + 2, 1u)] = (uint32_t)g;
+        off = hi;
+        segs += ns;
+    }
+    block_excl_scan(segs, wt, total);
+    if (threadIdx.x == 0) {
+        s.sums[nb + blockIdx.x] = total;
+        if (blockIdx.x == 0) {
+            s.total[0] = M;
+            s.total[3] = L;
+            s.offsets[s.Ks] = M;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256) k_plan_segments(SortPlanSets a) {
+    const SortPlanArgs& s = a.s[blockIdx.y];
+    const size_t base = (size_t)blockIdx.x * PLAN_BLOCK + threadIdx.x * 4;
+    if (blockIdx.x && (size_t)blockIdx.x * PLAN_BLOCK >= s.Ks) return;   // uniform across the block
+    __shared__ uint32_t wt[32];
+    const uint32_t nb = (s.Ks + PLAN_BLOCK - 1) / PLAN_BLOCK;
+    uint32_t S, total, v[4], sum = 0;
+    const uint32_t before = sums_before(s.sums + nb, blockIdx.x, nb, wt, S);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        v[j] = base + j < s.Ks ? s.counts[base + j] : 0;
+        sum += v[j];
+    }
+    uint32_t off = before + block_excl_scan(sum, wt, total);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        if (base + j >= s.Ks) break;
+        s.seg_base[base + j] = off;
+        off += v[j];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        s.total[1] = S;
+        s.seg_base[s.Ks] = S;
+    }
 }
 
 // One MSM of a multi-segment space, as the accumulate kernel reads it.
@@ -350,11 +435,11 @@ __device__ __forceinline__ void accumulate_chunks(const uint32_t* __restrict__ e
                                                   const uint32_t* __restrict__ seg_base, uint32_t K, uint32_t M,
                                                   uint32_t L, const uint4* __restrict__ bases, uint32_t base_offset,
                                                   uint32_t n_bases, uint4* __restrict__ partials,
-                                                  unsigned long long* __restrict__ work,
+                                                  unsigned long long* __restrict__ work, uint32_t per_block,
                                                   const MsmSegDev* __restrict__ segs = nullptr, uint32_t nsegs = 0) {
-    size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    size_t t = (size_t)blockIdx.x * per_block + threadIdx.x;
     size_t start = t * L;
-    const bool active = start < M;
+    const bool active = threadIdx.x < per_block && start < M;
     if (!LOCKSTEP && !active) return;
     size_t end = active ? (start + L < M ? start + L : M) : start;
     // last bucket g with offsets[g] <= start; then offsets[g+1] > start
@@ -431,6 +516,16 @@ __device__ __forceinline__ void accumulate_chunks(const uint32_t* __restrict__ e
 }
 
 constexpr int ACC_BLOCK_G1 = 512;   // lockstep block: 16 warps, one block per SM (<= 128 registers)
+
+// Chunks that a G1 accumulate block works on: all of its threads, or fewer, in
+// steps of a warp for each of the SM's four schedulers, when the chunks would
+// otherwise fill only some of the SMs.
+__device__ __forceinline__ uint32_t chunks_per_block(uint32_t M, uint32_t L) {
+    const uint32_t chunks = (uint32_t)(((uint64_t)M + L - 1) / L);
+    if (chunks >= MSM_SPREAD_THREADS) return ACC_BLOCK_G1;
+    constexpr uint32_t sms = MSM_SPREAD_THREADS / ACC_BLOCK_G1;
+    return ((chunks + sms - 1) / sms + 127) / 128 * 128;
+}
 constexpr int ACC_BLOCK_G2 = 128;
 // G2 accumulate blocks resident per SM that the register budget must allow
 // (1: the compiler may take 255 registers, which leaves room for 2)
@@ -477,9 +572,9 @@ __global__ void __launch_bounds__(ACC_BLOCK_G1, 1) k_accumulate_g1(const uint32_
                                                                    const uint4* __restrict__ bases, uint32_t base_offset,
                                                                    uint32_t n_bases, uint4* __restrict__ partials,
                                                                    unsigned long long* __restrict__ work) {
-    const uint32_t M = *d_M, L = *d_L;
-    if ((size_t)blockIdx.x * blockDim.x * L >= M) return;   // the whole block has no entries
-    accumulate_chunks<Fq, true>(entries, offsets, seg_base, K, M, L, bases, base_offset, n_bases, partials, work);
+    const uint32_t M = *d_M, L = *d_L, per = chunks_per_block(M, L);
+    if ((size_t)blockIdx.x * per * L >= M) return;   // the whole block has no entries
+    accumulate_chunks<Fq, true>(entries, offsets, seg_base, K, M, L, bases, base_offset, n_bases, partials, work, per);
 }
 
 __global__ void __launch_bounds__(ACC_BLOCK_G2, ACC_G2_MIN_BLOCKS) k_accumulate_g2(const uint32_t* __restrict__ entries,
@@ -491,7 +586,7 @@ __global__ void __launch_bounds__(ACC_BLOCK_G2, ACC_G2_MIN_BLOCKS) k_accumulate_
                                                                uint32_t n_bases, uint4* __restrict__ partials,
                                                                unsigned long long* __restrict__ work) {
     accumulate_chunks<Fq2, false>(entries, offsets, seg_base, K, *d_M, *d_L, bases, base_offset, n_bases, partials,
-                                  work);
+                                  work, blockDim.x);
 }
 
 __device__ __forceinline__ uint32_t n_partials(const uint32_t* offsets, uint32_t g, uint32_t L) {
@@ -872,9 +967,9 @@ __global__ void __launch_bounds__(ACC_BLOCK_G1, 1) k_accumulate_multi_g1(const u
                                                                          const MsmSegDev* __restrict__ segs,
                                                                          uint32_t nsegs, uint4* __restrict__ partials,
                                                                          unsigned long long* __restrict__ work) {
-    const uint32_t M = *d_M, L = *d_L;
-    if ((size_t)blockIdx.x * blockDim.x * L >= M) return;   // the whole block has no entries
-    accumulate_chunks<Fq, true, true>(entries, offsets, seg_base, K, M, L, nullptr, 0, 0, partials, work, segs,
+    const uint32_t M = *d_M, L = *d_L, per = chunks_per_block(M, L);
+    if ((size_t)blockIdx.x * per * L >= M) return;   // the whole block has no entries
+    accumulate_chunks<Fq, true, true>(entries, offsets, seg_base, K, M, L, nullptr, 0, 0, partials, work, per, segs,
                                       nsegs);
 }
 
@@ -887,7 +982,7 @@ __global__ void __launch_bounds__(ACC_BLOCK_G2, ACC_G2_MIN_BLOCKS) k_accumulate_
                                                                      uint32_t nsegs, uint4* __restrict__ partials,
                                                                      unsigned long long* __restrict__ work) {
     accumulate_chunks<Fq2, false, true>(entries, offsets, seg_base, K, *d_M, *d_L, nullptr, 0, 0, partials, work,
-                                        segs, nsegs);
+                                        blockDim.x, segs, nsegs);
 }
 
 // The bucket reduction of one segment of a space (msm_reduce_plan with one set).
@@ -1196,22 +1291,33 @@ static cudaError_t grow_bytes(cudaStream_t st, void*& p, size_t& cap, size_t nee
     return cudaSuccess;
 }
 
-// exclusive scan of in[0..len) into out[0..len] (out[len] = total); total also to *d_total
-static cudaError_t scan(const uint32_t* in, uint32_t* out, uint32_t len, uint32_t* tmp, uint32_t* d_total,
-                        cudaStream_t st) {
-    uint32_t nb = (len + 1023) / 1024;
-    if (nb == 0) nb = 1;
+// Scratch words for a plan over Ks buckets: two block sums each.
+static size_t plan_tmp_words(size_t Ks) { return 2 * ((Ks + PLAN_BLOCK - 1) / PLAN_BLOCK); }
+
+// The accumulate's plan from the bucket counts of `count` sorts (d_counts
+// filled); the scatter follows.
+static cudaError_t sort_plan(MsmSort* const* sorts, int count, cudaStream_t st) {
+    SortPlanSets a = {};
+    a.wave = accumulate_wave();
+    uint32_t nb = 1;
+    for (int j = 0; j < count; j++) {
+        const MsmSort& s = *sorts[j];
+        a.s[j] = {s.d_counts, s.d_offsets, s.d_cursor, s.d_seg_base, s.d_fat_list, s.d_scan_tmp, s.d_total, s.Ks, s.K,
+                  s.chunk};
+        nb = std::max(nb, (s.Ks + PLAN_BLOCK - 1) / PLAN_BLOCK);
+    }
+    const dim3 grid(nb, count);
     {
-        TimedLaunch tl("msm_scan", st);
-        k_scan_blocks<<<nb, 256, 0, st>>>(in, out, len, tmp);
+        TimedLaunch tl("msm_plan", st);
+        k_plan_sums<<<grid, 256, 0, st>>>(a);
     }
     {
-        TimedLaunch tl("msm_scan", st);
-        k_scan_top<<<1, 1024, 0, st>>>(tmp, nb, d_total);
+        TimedLaunch tl("msm_plan", st);
+        k_plan_offsets<<<grid, 256, 0, st>>>(a);
     }
     {
-        TimedLaunch tl("msm_scan", st);
-        k_scan_add<<<blocks_for(len ? len : 1, 256), 256, 0, st>>>(out, len, tmp, d_total);
+        TimedLaunch tl("msm_plan", st);
+        k_plan_segments<<<grid, 256, 0, st>>>(a);
     }
     return cudaGetLastError();
 }
@@ -1235,9 +1341,9 @@ cudaError_t msm_sort(MsmSort& s, const void* d_scalars, size_t n, bool montgomer
         set_error("MSM of %zu points x %d windows exceeds the 2^31 entry-index limit", n, s.W);
         return cudaErrorInvalidValue;
     }
-    // the smallest chunk the accumulate may use (buffers are sized for it);
-    // the one it does use is chosen on the device from the entry count (k_nseg)
-    s.chunk = 16;
+    // the smallest chunk the accumulate may use (fixed scratch is sized for 16);
+    // the one it does use is chosen on the device from the entry count
+    s.chunk = s.fixed ? 16 : MSM_MIN_CHUNK;
     const uint32_t kw = shared_windows ? 0u : s.B, ew = shared_windows ? (uint32_t)n : 0u;
     const uint32_t sink = constant_work ? s.K : NO_KEY;
     size_t nn = n ? n : 1;
@@ -1258,7 +1364,7 @@ cudaError_t msm_sort(MsmSort& s, const void* d_scalars, size_t n, bool montgomer
         G16_CUDA(grow(st, s.d_fat_list, cap, kk));
         s.cap_k = cap;
     }
-    G16_CUDA(grow(st, s.d_scan_tmp, s.cap_tmp, kk / 1024 + 2, s.fixed));
+    G16_CUDA(grow(st, s.d_scan_tmp, s.cap_tmp, plan_tmp_words(s.Ks), s.fixed));
     G16_CUDA(grow(st, s.d_entries, s.cap_entries, nn * s.W, s.fixed));
     if (!s.d_total) {
         if (s.fixed) G16_CUDA(fixed_too_small(4 * sizeof(uint32_t), 0));
@@ -1266,32 +1372,31 @@ cudaError_t msm_sort(MsmSort& s, const void* d_scalars, size_t n, bool montgomer
     }
 
     G16_CUDA(cudaMemsetAsync(s.d_counts, 0, kk * sizeof(uint32_t), st));
-    G16_CUDA(cudaMemsetAsync(s.d_total, 0, 4 * sizeof(uint32_t), st));
     if (n) {
         timer().add_bytes("msm_digits", 64.0 * n);   // scalars in, standard-form copy out
         TimedLaunch tl("msm_digits", st);
-        k_digits_count<<<blocks_for(n, 256), 256, 0, st>>>((const uint4*)d_scalars, montgomery ? 1 : 0, (uint32_t)n,
-                                                          c, s.W, kw, sink, (uint4*)s.d_scalars_std, s.d_counts);
+        if (n < DIGITS_SPLIT)
+            k_digits_count<8><<<blocks_for(n, 32), 256, 0, st>>>((const uint4*)d_scalars, montgomery ? 1 : 0,
+                                                               (uint32_t)n, c, s.W, kw, sink,
+                                                               (uint4*)s.d_scalars_std, s.d_counts);
+        else
+            k_digits_count<1><<<blocks_for(n, 256), 256, 0, st>>>((const uint4*)d_scalars, montgomery ? 1 : 0,
+                                                                (uint32_t)n, c, s.W, kw, sink,
+                                                                (uint4*)s.d_scalars_std, s.d_counts);
     }
     G16_CUDA(cudaGetLastError());
-    G16_CUDA(scan(s.d_counts, s.d_offsets, s.Ks, s.d_scan_tmp, s.d_total, st));
-    {
-        TimedLaunch tl("msm_copy", st);
-        k_copy_u32<<<blocks_for(s.Ks, 256), 256, 0, st>>>(s.d_cursor, s.d_offsets, s.Ks);
-    }
+    MsmSort* const one[1] = {&s};
+    G16_CUDA(sort_plan(one, 1, st));
     if (n) {
         TimedLaunch tl("msm_scatter", st);
-        k_scatter<<<blocks_for(n, 256), 256, 0, st>>>((const uint4*)s.d_scalars_std, (uint32_t)n, c, s.W, kw, ew,
-                                                     sink, s.d_cursor, s.d_entries);
+        if (n < DIGITS_SPLIT)
+            k_scatter<8><<<blocks_for(n, 32), 256, 0, st>>>((const uint4*)s.d_scalars_std, (uint32_t)n, c, s.W, kw, ew,
+                                                          sink, s.d_cursor, s.d_entries);
+        else
+            k_scatter<1><<<blocks_for(n, 256), 256, 0, st>>>((const uint4*)s.d_scalars_std, (uint32_t)n, c, s.W, kw,
+                                                           ew, sink, s.d_cursor, s.d_entries);
     }
     G16_CUDA(cudaGetLastError());
-    // per-bucket segment counts -> segment base (into counts, then scanned)
-    {
-        TimedLaunch tl("msm_nseg", st);
-        k_nseg<<<blocks_for(s.Ks, 256), 256, 0, st>>>(s.d_offsets, s.Ks, s.K, s.chunk, accumulate_wave(),
-                                                       s.d_counts, s.d_fat_list, s.d_total + 2, s.d_total);
-    }
-    G16_CUDA(scan(s.d_counts, s.d_seg_base, s.Ks, s.d_scan_tmp, s.d_total + 1, st));
     return cudaSuccess;
 }
 
@@ -1321,7 +1426,7 @@ cudaError_t msm_sort_sets(MsmSort* sorts, const MsmLiveSets& sets, const void* d
         s.constant_work = constant_work;
         s.Ks = s.K + (constant_work ? 1u : 0u);
         s.n = sets.rows[j];
-        s.chunk = 16;
+        s.chunk = MSM_MIN_CHUNK;
         if ((size_t)sets.rows[j] * (size_t)W >= 0x80000000ull || sets.rows[j] > n) {
             set_error("live set of %u rows x %d windows exceeds the 2^31 entry-index limit", sets.rows[j], W);
             return cudaErrorInvalidValue;
@@ -1340,11 +1445,10 @@ cudaError_t msm_sort_sets(MsmSort* sorts, const MsmLiveSets& sets, const void* d
             G16_CUDA(grow(st, s.d_fat_list, cap, kk));
             s.cap_k = cap;
         }
-        G16_CUDA(grow(st, s.d_scan_tmp, s.cap_tmp, kk / 1024 + 2));
+        G16_CUDA(grow(st, s.d_scan_tmp, s.cap_tmp, plan_tmp_words(s.Ks)));
         G16_CUDA(grow(st, s.d_entries, s.cap_entries, (size_t)(sets.rows[j] ? sets.rows[j] : 1) * W));
         if (!s.d_total) G16_CUDA(g16::dev_realloc_async(&s.d_total, 4 * sizeof(uint32_t), st, false));
         G16_CUDA(cudaMemsetAsync(s.d_counts, 0, kk * sizeof(uint32_t), st));
-        G16_CUDA(cudaMemsetAsync(s.d_total, 0, 4 * sizeof(uint32_t), st));
         a.rank[j] = sets.d_rank[j];
         a.counts[j] = s.d_counts;
         a.cursor[j] = s.d_cursor;
@@ -1359,33 +1463,37 @@ cudaError_t msm_sort_sets(MsmSort* sorts, const MsmLiveSets& sets, const void* d
     if (n) {
         timer().add_bytes("msm_digits", 64.0 * n);   // scalars in, standard-form copy out
         TimedLaunch tl("msm_digits", st);
-        k_digits_count_sets<<<blocks_for(n, 256), 256, 0, st>>>((const uint4*)d_scalars, montgomery ? 1 : 0,
-                                                               (uint32_t)n, c, W, sink, sets.count, a,
-                                                               (uint4*)s0.d_scalars_std);
+        if (n < DIGITS_SPLIT)
+            k_digits_count_sets<8><<<blocks_for(n, 32), 256, 0, st>>>((const uint4*)d_scalars, montgomery ? 1 : 0,
+                                                                    (uint32_t)n, c, W, sink, sets.count, a,
+                                                                    (uint4*)s0.d_scalars_std);
+        else
+            k_digits_count_sets<1><<<blocks_for(n, 256), 256, 0, st>>>((const uint4*)d_scalars, montgomery ? 1 : 0,
+                                                                     (uint32_t)n, c, W, sink, sets.count, a,
+                                                                     (uint4*)s0.d_scalars_std);
     }
     G16_CUDA(cudaGetLastError());
-    for (int j = 0; j < sets.count; j++) {
-        MsmSort& s = sorts[j];
-        G16_CUDA(scan(s.d_counts, s.d_offsets, s.Ks, s.d_scan_tmp, s.d_total, st));
-        TimedLaunch tl("msm_copy", st);
-        k_copy_u32<<<blocks_for(s.Ks, 256), 256, 0, st>>>(s.d_cursor, s.d_offsets, s.Ks);
-    }
+    MsmSort* all[MSM_MAX_SETS] = {};
+    for (int j = 0; j < sets.count; j++) all[j] = &sorts[j];
+    G16_CUDA(sort_plan(all, sets.count, st));
     if (n) {
         TimedLaunch tl("msm_scatter", st);
-        k_scatter_sets<<<blocks_for(n, 256), 256, 0, st>>>((const uint4*)s0.d_scalars_std, (uint32_t)n, c, W, sink,
-                                                          sets.count, a);
+        if (n < DIGITS_SPLIT)
+            k_scatter_sets<8><<<blocks_for(n, 32), 256, 0, st>>>((const uint4*)s0.d_scalars_std, (uint32_t)n, c, W, sink,
+                                                               sets.count, a);
+        else
+            k_scatter_sets<1><<<blocks_for(n, 256), 256, 0, st>>>((const uint4*)s0.d_scalars_std, (uint32_t)n, c, W,
+                                                                sink, sets.count, a);
     }
     G16_CUDA(cudaGetLastError());
-    for (int j = 0; j < sets.count; j++) {
-        MsmSort& s = sorts[j];
-        {
-            TimedLaunch tl("msm_nseg", st);
-            k_nseg<<<blocks_for(s.Ks, 256), 256, 0, st>>>(s.d_offsets, s.Ks, s.K, s.chunk, accumulate_wave(),
-                                                           s.d_counts, s.d_fat_list, s.d_total + 2, s.d_total);
-        }
-        G16_CUDA(scan(s.d_counts, s.d_seg_base, s.Ks, s.d_scan_tmp, s.d_total + 1, st));
-    }
     return cudaSuccess;
+}
+
+// Blocks of a G1 accumulate over up to `chunks` chunks: enough for whole blocks
+// of chunks, and for the spread ones (chunks_per_block), one per SM at most.
+static unsigned accumulate_blocks_g1(size_t chunks) {
+    const unsigned spread = std::min<unsigned>(MSM_SPREAD_THREADS / ACC_BLOCK_G1, blocks_for(chunks, 128));
+    return std::max(blocks_for(chunks, ACC_BLOCK_G1), spread);
 }
 
 // threads of a k_reduce_sets block: a group per point of a term (nb a power of
@@ -1400,7 +1508,7 @@ template <class F>
 static cudaError_t accumulate(const MsmSort& s, MsmAccum& acc, const void* d_bases, uint32_t base_offset,
                               uint32_t n_bases, cudaStream_t st, size_t xyzz_bytes, const char* tag) {
     size_t max_entries = (s.n ? s.n : 1) * (size_t)s.W;
-    size_t chunks = (max_entries + s.chunk - 1) / s.chunk;
+    const size_t chunks = msm_max_chunks(max_entries, s.chunk);
     size_t max_partials = (size_t)s.Ks + chunks + 1;
     G16_CUDA(grow_bytes(st, acc.d_partials, acc.cap_partials, max_partials * xyzz_bytes, acc.fixed));
     const uint32_t Wr = s.shared ? 1u : (uint32_t)s.W;   // bucket sets to reduce
@@ -1423,7 +1531,7 @@ static cudaError_t accumulate(const MsmSort& s, MsmAccum& acc, const void* d_bas
     {
         TimedLaunch tl(tag, st);
         if (std::is_same<F, g16d::Fq>::value)
-            k_accumulate_g1<<<blocks_for(chunks, ACC_BLOCK_G1), ACC_BLOCK_G1, 0, st>>>(
+            k_accumulate_g1<<<accumulate_blocks_g1(chunks), ACC_BLOCK_G1, 0, st>>>(
                 s.d_entries, s.d_offsets, s.d_seg_base, s.Ks, s.d_total, s.d_total + 3, (const uint4*)d_bases,
                 base_offset, n_bases, partials, acc.d_work);
         else
@@ -1559,7 +1667,7 @@ cudaError_t msm_batch_setup(MsmSources& so, MsmSpace* const* spaces, int nspaces
         s.K = s.Ks = sp.K;
         s.B = 0;
         s.shared = true;
-        s.chunk = 16;
+        s.chunk = MSM_MIN_CHUNK;
         s.n = sp.max_entries;   // accumulate sizes its partials by entries, W = 1 below
         s.W = 1;
         const size_t kk = (size_t)sp.K + 1;
@@ -1576,11 +1684,11 @@ cudaError_t msm_batch_setup(MsmSources& so, MsmSpace* const* spaces, int nspaces
             G16_CUDA(grow(st, s.d_fat_list, cap, kk));
             s.cap_k = cap;
         }
-        G16_CUDA(grow(st, s.d_scan_tmp, s.cap_tmp, kk / 1024 + 2));
+        G16_CUDA(grow(st, s.d_scan_tmp, s.cap_tmp, plan_tmp_words(s.Ks)));
         G16_CUDA(grow(st, s.d_entries, s.cap_entries, sp.max_entries ? sp.max_entries : 1));
         if (!s.d_total) G16_CUDA(g16::dev_realloc_async(&s.d_total, 4 * sizeof(uint32_t), st, false));
         MsmAccum& a = sp.acc;
-        const size_t chunks = (sp.max_entries + s.chunk - 1) / s.chunk;
+        const size_t chunks = msm_max_chunks(sp.max_entries, s.chunk);
         G16_CUDA(grow_bytes(st, a.d_partials, a.cap_partials, ((size_t)sp.K + chunks + 1) * pb));
         G16_CUDA(grow_bytes(st, a.d_buckets, a.cap_buckets, ((size_t)sp.K + 1) * pb));
         G16_CUDA(grow_bytes(st, a.d_segments, a.cap_segments, (out_block + 1) * pb));
@@ -1632,7 +1740,6 @@ cudaError_t msm_batch_sort(MsmSources& so, MsmSpace* const* spaces, int nspaces,
     for (int i = 0; i < nspaces; i++) {
         MsmSort& s = spaces[i]->sort;
         G16_CUDA(cudaMemsetAsync(s.d_counts, 0, ((size_t)s.K + 1) * sizeof(uint32_t), st));
-        G16_CUDA(cudaMemsetAsync(s.d_total, 0, 4 * sizeof(uint32_t), st));
     }
     const uint32_t nsrc = (uint32_t)so.srcs.size();
     if (so.total_blocks) {
@@ -1640,27 +1747,18 @@ cudaError_t msm_batch_sort(MsmSources& so, MsmSpace* const* spaces, int nspaces,
         k_digits_multi<<<so.total_blocks, 256, 0, st>>>((const MsmSourceDev*)so.d_desc, so.d_blk, nsrc);
     }
     G16_CUDA(cudaGetLastError());
-    for (int i = 0; i < nspaces; i++) {
-        MsmSort& s = spaces[i]->sort;
-        G16_CUDA(scan(s.d_counts, s.d_offsets, s.K, s.d_scan_tmp, s.d_total, st));
-        TimedLaunch tl("msm_copy", st);
-        k_copy_u32<<<blocks_for(s.K ? s.K : 1, 256), 256, 0, st>>>(s.d_cursor, s.d_offsets, s.K);
+    MsmSort* all[MSM_MAX_SETS] = {};
+    if (nspaces > MSM_MAX_SETS) {
+        set_error("%d MSM spaces in one sort (at most %d)", nspaces, MSM_MAX_SETS);
+        return cudaErrorInvalidValue;
     }
+    for (int i = 0; i < nspaces; i++) all[i] = &spaces[i]->sort;
+    G16_CUDA(sort_plan(all, nspaces, st));
     if (so.total_blocks) {
         TimedLaunch tl("msm_scatter", st);
         k_scatter_multi<<<so.total_blocks, 256, 0, st>>>((const MsmSourceDev*)so.d_desc, so.d_blk, nsrc);
     }
     G16_CUDA(cudaGetLastError());
-    for (int i = 0; i < nspaces; i++) {
-        MsmSort& s = spaces[i]->sort;
-        {
-            TimedLaunch tl("msm_nseg", st);
-            k_nseg<<<blocks_for(s.K ? s.K : 1, 256), 256, 0, st>>>(s.d_offsets, s.K, s.K, s.chunk, accumulate_wave(),
-                                                                   s.d_counts, s.d_fat_list, s.d_total + 2,
-                                                                   s.d_total);
-        }
-        G16_CUDA(scan(s.d_counts, s.d_seg_base, s.K, s.d_scan_tmp, s.d_total + 1, st));
-    }
     return cudaSuccess;
 }
 
@@ -1668,7 +1766,7 @@ template <class F, int LB>
 static cudaError_t space_accumulate(MsmSpace& sp, cudaStream_t st, size_t xyzz_bytes, const char* tag) {
     MsmSort& s = sp.sort;
     MsmAccum& a = sp.acc;
-    const size_t chunks = (sp.max_entries + s.chunk - 1) / s.chunk;
+    const size_t chunks = msm_max_chunks(sp.max_entries, s.chunk);
     G16_CUDA(cudaMemsetAsync(a.d_work, 0, sizeof(unsigned long long), st));
     uint4* partials = (uint4*)a.d_partials;
     const uint32_t nsegs = (uint32_t)sp.segs.size();
@@ -1681,7 +1779,7 @@ static cudaError_t space_accumulate(MsmSpace& sp, cudaStream_t st, size_t xyzz_b
     if (chunks) {
         TimedLaunch tl(tag, st);
         if (std::is_same<F, g16d::Fq>::value)
-            k_accumulate_multi_g1<<<blocks_for(chunks, ACC_BLOCK_G1), ACC_BLOCK_G1, 0, st>>>(
+            k_accumulate_multi_g1<<<accumulate_blocks_g1(chunks), ACC_BLOCK_G1, 0, st>>>(
                 s.d_entries, s.d_offsets, s.d_seg_base, s.K, s.d_total, s.d_total + 3, (const MsmSegDev*)sp.d_segdev,
                 nsegs, partials, a.d_work);
         else

@@ -69,8 +69,7 @@ constexpr uint64_t msm_reduce_pieces(bool shared_windows) {
 // blocks spread the pieces over the SMs, and the blocks' terms are summed in
 // parallel by the second kernel.  Against one thread per piece in blocks of 2^8
 // (about 250 registers): the five reductions of a 1.1M-constraint prove 2.41 ->
-// 1.11 ms, of a 2^15-constraint one 1.39 -> 0.64 ms, of a 500-constraint one
-// 0.77 -> 0.21 ms (serialised).
+// 1.11 ms, of a 500-constraint one 0.77 -> 0.21 ms (serialised).
 #ifndef G16_REDUCE_LB_G1
 #define G16_REDUCE_LB_G1 5
 #endif
@@ -149,6 +148,18 @@ inline MsmSpaceReduceLayout msm_space_reduce_layout(const std::vector<uint32_t>&
     return L;
 }
 
+// Accumulate chunks (sorted entries per thread): 16 or more, or down to
+// MSM_MIN_CHUNK when 16 would leave SMs without their 512 threads (min_chunk in
+// msm.cu).  Buffers hold the most chunks any entry count up to the maximum can
+// give.
+constexpr uint32_t MSM_MIN_CHUNK = 4;
+constexpr uint32_t MSM_SPREAD_THREADS = 148 * 512;
+constexpr size_t msm_max_chunks(size_t max_entries, uint32_t floor) {
+    const size_t whole = (max_entries + 15) / 16, least = (max_entries + floor - 1) / floor;
+    const size_t spread = least < MSM_SPREAD_THREADS ? least : MSM_SPREAD_THREADS;
+    return whole > spread ? whole : spread;
+}
+
 struct MsmSort {
     // parameters
     int c = 0, W = 0;
@@ -159,7 +170,7 @@ struct MsmSort {
     bool constant_work = false;   // zero digits are sorted into the sink bucket K
     uint64_t reduce_pieces = 0;   // bucket-reduction piece target; 0: msm_reduce_pieces(shared)
     size_t n = 0;          // scalars sorted
-    uint32_t chunk = 16;   // smallest accumulate chunk (buffers are sized for it)
+    uint32_t chunk = 16;   // smallest accumulate chunk
     // device buffers (capacities in elements)
     uint32_t* d_scalars_std = nullptr;  size_t cap_scalars = 0;   // 8 u32 per scalar
     uint32_t* d_counts = nullptr;       size_t cap_k = 0;         // K + 1
@@ -169,7 +180,7 @@ struct MsmSort {
     uint32_t* d_fat_list = nullptr;                               // buckets with many partials
     uint32_t* d_scan_tmp = nullptr;     size_t cap_tmp = 0;
     uint32_t* d_entries = nullptr;      size_t cap_entries = 0;
-    uint32_t* d_total = nullptr;                                  // [0] = M, [1] = S, [2] = fat buckets, [3] = L
+    uint32_t* d_total = nullptr;                                  // [0] = M, [1] = partial sums, [2] = fat buckets, [3] = L
     // the buffers are views into memory the struct does not own (the
     // allocation-free entry point's fixed scratch): a buffer too small for a
     // call is an error, never a cudaFree and cudaMalloc

@@ -268,8 +268,9 @@ uint64_t workspace_estimate(uint64_t nv, uint64_t n, int c_w, int c_h, uint64_t 
     const uint64_t Kw = (1ull << (c_w - 1)) * (tables ? 1 : Ww), Kh = (1ull << (c_h - 1)) * (tables ? 1 : Wh);
     uint64_t b = nv * 32 + n * 32 * 4;
     b += nv * 32 + (ra + rb + rl) * Ww * 4 + 3 * 24 * (Kw + 1) + n * 32 + n * Wh * 4 + 24 * (Kh + 1);
-    b += 128 * (3 * Kw * 2 + (ra + rb + rl) * Ww / 16 + 3) + 256 * (Kw * 2 + rb * Ww / 16 + 1);
-    b += 128 * (Kh * 2 + n * Wh / 16 + 1) + (16ull << 20);
+    auto chunks = [](uint64_t entries) { return (uint64_t)msm_max_chunks(entries, MSM_MIN_CHUNK) + 1; };
+    b += 128 * (3 * Kw * 2 + chunks(ra * Ww) + chunks(rb * Ww) + chunks(rl * Ww)) + 256 * (Kw * 2 + chunks(rb * Ww));
+    b += 128 * (Kh * 2 + chunks(n * Wh)) + (16ull << 20);
     return b;
 }
 
