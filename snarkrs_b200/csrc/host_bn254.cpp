@@ -75,6 +75,23 @@ void batch_to_affine(const Jac<F>* in, Affine<F>* out, size_t n) {
     }
 }
 
+template <class F>
+std::vector<Affine<F>> fixed_base_table(const Affine<F>& p) {
+    std::vector<Jac<F>> t(8 * RADIX16_DIGITS);
+    Jac<F> b = Jac<F>::from_affine(p);
+    for (int i = 0; i < RADIX16_DIGITS; i++) {
+        Jac<F>* row = &t[8 * i];
+        row[0] = b;
+        for (int j = 1; j < 8; j++) row[j] = j == 1 ? b.dbl() : row[j - 1] + b;
+        b = row[7].dbl();
+    }
+    std::vector<Affine<F>> out(t.size());
+    batch_to_affine(t.data(), out.data(), t.size());
+    return out;
+}
+
+template std::vector<Affine<Fq>> fixed_base_table<Fq>(const Affine<Fq>&);
+template std::vector<Affine<Fq2>> fixed_base_table<Fq2>(const Affine<Fq2>&);
 template void batch_to_affine<Fq>(const Jac<Fq>*, Affine<Fq>*, size_t);
 template void batch_to_affine<Fq2>(const Jac<Fq2>*, Affine<Fq2>*, size_t);
 

@@ -438,23 +438,20 @@ G1J g1_mul(const G1J& p, const g16::Fr& k) {
     k.to_std(s);
     return p.mul(s);
 }
-G2J g2_mul(const G2J& p, const g16::Fr& k) {
-    uint64_t s[4];
-    k.to_std(s);
-    return p.mul(s);
-}
-
 }  // namespace
 
 namespace g16 {
 
 BlinderTerms blinder_terms(const g16_circuit* c, const g16::Fr& r, const g16::Fr& s) {
     BlinderTerms t;
-    G1J d1 = G1J::from_affine(c->delta1);
-    t.d1r = g1_mul(d1, r);
-    t.d1s = g1_mul(d1, s);
-    t.d1rs = g1_mul(d1, r * s);
-    t.d2s = g2_mul(G2J::from_affine(c->delta2), s);
+    uint64_t kr[4], ks[4], krs[4];
+    r.to_std(kr);
+    s.to_std(ks);
+    (r * s).to_std(krs);
+    t.d1r = fixed_base_mul(c->delta1_table, kr);
+    t.d1s = fixed_base_mul(c->delta1_table, ks);
+    t.d1rs = fixed_base_mul(c->delta1_table, krs);
+    t.d2s = fixed_base_mul(c->delta2_table, ks);
     return t;
 }
 
@@ -463,7 +460,10 @@ void assemble(const g16_circuit* c, const MsmJac& m, const BlinderTerms& t, cons
     G1J pi_a = m.a.add_affine(c->alpha1) + t.d1r;
     G2J pi_b = m.b2.add_affine(c->beta2) + t.d2s;
     G1J pib1 = m.b1.add_affine(c->beta1) + t.d1s;
-    G1J pi_c = m.l + m.h + g1_mul(pi_a, s) + g1_mul(pib1, r) + t.d1rs.neg();
+    uint64_t kr[4], ks[4];
+    r.to_std(kr);
+    s.to_std(ks);
+    G1J pi_c = m.l + m.h + mul_pair(pi_a, ks, pib1, kr) + t.d1rs.neg();
     G1J g1s[2] = {pi_a, pi_c};
     G1A g1a[2];
     batch_to_affine(g1s, g1a, 2);
@@ -1280,6 +1280,8 @@ int g16_prepare(g16_backend* b, const g16_zkey_view* k, g16_circuit** out) {
         return fail(G16_ERR_BACKEND, "non-canonical header point");
     if (c->alpha1.inf || c->beta1.inf || c->delta1.inf || c->beta2.inf || c->delta2.inf)
         return fail(G16_ERR_BACKEND, "a header point is the point at infinity");
+    c->delta1_table = fixed_base_table(c->delta1);
+    c->delta2_table = fixed_base_table(c->delta2);
     if (k->gamma_g2 && !unpack(c->gamma2, k->gamma_g2)) return fail(G16_ERR_BACKEND, "non-canonical gamma_g2");
     if (!k->gamma_g2) c->gamma2.inf = true;
     if (k->ic) {

@@ -134,6 +134,8 @@ struct g16_circuit {
     g16::NttTables ntt;
     g16::G1A alpha1, beta1, delta1;
     g16::G2A beta2, delta2, gamma2;
+    std::vector<g16::G1A> delta1_table;     // multiples of delta for the blinders' products
+    std::vector<g16::G2A> delta2_table;
     std::vector<g16::G1A> ic;               // verifying key: constant wire, then the public inputs
     // workspaces: one per proof in flight
     std::mutex mu;
