@@ -123,8 +123,8 @@ __device__ __forceinline__ Xyzz<F> xyzz_add_affine(const Xyzz<F>& p, const F& x2
         r.zz = mul(p.zz, pp);
         r.zzz = mul(p.zzz, ppp);
     } else {
-        F pp, rr2, ppp, q, t, ypp;
-        fmul2<INL>(pp_, pp_, rr, rr, pp, rr2);
+        F ppp, q, t, ypp;
+        const F pp = fsqr<INL>(pp_), rr2 = fsqr<INL>(rr);
         fmul2<INL>(pp_, pp, p.x, pp, ppp, q);
         r.x = sub(sub(rr2, ppp), dbl(q));
         fmul3<INL>(rr, sub(q, r.x), p.y, ppp, p.zzz, ppp, t, ypp, r.zzz);

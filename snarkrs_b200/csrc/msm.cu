@@ -258,7 +258,7 @@ __device__ __forceinline__ uint32_t fat_job_len(uint32_t ns) {
 // partial sums and only skewed buckets (a repeated scalar such as 1) take the
 // fat-bucket path.  Sparse scalars (witnesses of zeros and ones) still spread
 // over the whole GPU.  Last, the chunks are fitted to whole waves of `wave`
-// threads (one 512-thread G1 block per SM) when that saves 5% or more: a
+// threads (the G1 accumulate's 512 threads an SM) when that saves 5% or more: a
 // launch takes about (waves x L) additions per thread, so 2.4 waves of 16
 // entries lose to 2 waves of 20 (a sparse witness MSM of the 2^21 prove).
 constexpr uint32_t ACC_THREADS = 1u << 19;
@@ -421,41 +421,35 @@ struct MsmSegDev {
 };
 
 // ---- accumulate: one thread per chunk of L sorted entries ----
-// LOCKSTEP: a block-wide barrier after every entry keeps the block's warps on
-// the same instructions.  A fully inlined G1 madd is too long for the
-// instruction cache, and warps that drift apart stall on instruction fetch
-// (ncu: no_instruction was the top stall); in lockstep, one fetch serves the
-// whole block.  G2 calls out-of-line Fq2 products and runs without it.
+// Bound by the issue of wide multiply-adds (1232 for a G1 mixed addition, 3200
+// for a G2 one): 6.7 G G1 additions/s in a 2^20 MSM, 0.89 of the rate at which
+// an SM issues them.  Warps run freely; a block-wide barrier after every entry,
+// which kept a longer body in the instruction cache, costs 12% now.
 // MULTI: the buckets belong to several MSMs (segments, msm_space_*), each
 // with its own base table; the segment of bucket g is the last one whose
 // key_start is <= g, followed forward as g grows.
-template <class F, bool LOCKSTEP, bool MULTI = false>
+template <class F, bool MULTI = false>
 __device__ __forceinline__ void accumulate_chunks(const uint32_t* __restrict__ entries,
                                                   const uint32_t* __restrict__ offsets,
                                                   const uint32_t* __restrict__ seg_base, uint32_t K, uint32_t M,
                                                   uint32_t L, const uint4* __restrict__ bases, uint32_t base_offset,
                                                   uint32_t n_bases, uint4* __restrict__ partials,
-                                                  unsigned long long* __restrict__ work, uint32_t per_block,
+                                                  unsigned long long* __restrict__ work,
                                                   const MsmSegDev* __restrict__ segs = nullptr, uint32_t nsegs = 0) {
-    size_t t = (size_t)blockIdx.x * per_block + threadIdx.x;
-    size_t start = t * L;
-    const bool active = threadIdx.x < per_block && start < M;
-    if (!LOCKSTEP && !active) return;
-    size_t end = active ? (start + L < M ? start + L : M) : start;
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, start = t * L;
+    if (start >= M) return;
+    const size_t end = start + L < M ? start + L : M;
     // last bucket g with offsets[g] <= start; then offsets[g+1] > start
-    uint32_t g = 0, next = 0;
-    if (active) {
-        uint32_t lo = 0, hi = K;
-        while (hi - lo > 1) {
-            uint32_t mid = (lo + hi) >> 1;
-            if (offsets[mid] <= start) lo = mid; else hi = mid;
-        }
-        g = lo;
-        next = offsets[g + 1];
+    uint32_t lo = 0, hi = K;
+    while (hi - lo > 1) {
+        uint32_t mid = (lo + hi) >> 1;
+        if (offsets[mid] <= start) lo = mid; else hi = mid;
     }
+    uint32_t g = lo, next = offsets[g + 1];
     uint32_t si = 0, seg_end = 0xffffffffu;
-    if (MULTI && active) {
-        uint32_t lo = 0, hi = nsegs;
+    if (MULTI) {
+        lo = 0;
+        hi = nsegs;
         while (hi - lo > 1) {
             uint32_t mid = (lo + hi) >> 1;
             if (segs[mid].key_start <= g) lo = mid; else hi = mid;
@@ -468,70 +462,57 @@ __device__ __forceinline__ void accumulate_chunks(const uint32_t* __restrict__ e
     }
     Xyzz<F> acc = Xyzz<F>::identity();
     unsigned adds = 0;
-    const size_t stop = LOCKSTEP ? start + L : end;   // lockstep: every thread runs L steps
-    for (size_t k = start; k < stop; k++) {
-        if (!LOCKSTEP || k < end) {
-            if (k == next) {
-                st_xyzz<F>(partials, seg_base[g] + (uint32_t)(t - offsets[g] / L), acc);
-                acc = Xyzz<F>::identity();
-                do {
-                    g++;
-                    next = offsets[g + 1];
-                } while (next <= k);
-                if (MULTI) {
-                    while (g >= seg_end) {
-                        si++;
-                        bases = segs[si].bases;
-                        n_bases = segs[si].n_bases;
-                        seg_end = si + 1 < nsegs ? segs[si + 1].key_start : 0xffffffffu;
-                    }
-                }
-            }
-            uint32_t e = entries[k];
-            if (k + 1 < end) {   // bring the next entry's base towards L1 while this one is added
-                uint32_t nx = (entries[k + 1] & 0x7fffffffu) - base_offset;
-                if (nx < n_bases)
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(bases + (size_t)nx * (2 * Codec<F>::U4)));
-            }
-            uint32_t idx = e & 0x7fffffffu;
-            if (idx >= base_offset && idx - base_offset < n_bases) {
-                Affine<F> p = ld_affine<F>(bases, idx - base_offset);
-                if (!p.is_inf()) {
-                    if (e >> 31) p.y = neg(p.y);
-                    // G1 keeps its products inlined; the Fq2 body is large enough
-                    // that one out-of-line Fq2 product (three Fq chains) runs
-                    // faster than inlined code that misses the instruction cache
-                    acc = xyzz_add_affine<F, !std::is_same<F, Fq2>::value>(acc, p.x, p.y);
-                    adds++;
+    for (size_t k = start; k < end; k++) {
+        if (k == next) {
+            st_xyzz<F>(partials, seg_base[g] + (uint32_t)(t - offsets[g] / L), acc);
+            acc = Xyzz<F>::identity();
+            do {
+                g++;
+                next = offsets[g + 1];
+            } while (next <= k);
+            if (MULTI) {
+                while (g >= seg_end) {
+                    si++;
+                    bases = segs[si].bases;
+                    n_bases = segs[si].n_bases;
+                    seg_end = si + 1 < nsegs ? segs[si + 1].key_start : 0xffffffffu;
                 }
             }
         }
-        if (LOCKSTEP) __syncthreads();
+        uint32_t e = entries[k];
+        if (k + 1 < end) {   // bring the next entry's base towards L1 while this one is added
+            uint32_t nx = (entries[k + 1] & 0x7fffffffu) - base_offset;
+            if (nx < n_bases)
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(bases + (size_t)nx * (2 * Codec<F>::U4)));
+        }
+        uint32_t idx = e & 0x7fffffffu;
+        if (idx >= base_offset && idx - base_offset < n_bases) {
+            Affine<F> p = ld_affine<F>(bases, idx - base_offset);
+            if (!p.is_inf()) {
+                if (e >> 31) p.y = neg(p.y);
+                // G1 keeps its products inlined; the Fq2 body is large enough
+                // that one out-of-line Fq2 product (three Fq chains) runs
+                // faster than inlined code that misses the instruction cache
+                // (G2 MSM 2^18: 2.18 against 2.44 ms)
+                acc = xyzz_add_affine<F, !std::is_same<F, Fq2>::value>(acc, p.x, p.y);
+                adds++;
+            }
+        }
     }
-    if (active) st_xyzz<F>(partials, seg_base[g] + (uint32_t)(t - offsets[g] / L), acc);
-    // mixed additions performed, one atomic per warp (every lane reaches here in lockstep mode)
+    st_xyzz<F>(partials, seg_base[g] + (uint32_t)(t - offsets[g] / L), acc);
+    // mixed additions performed, one atomic per warp
     unsigned mask = __activemask();
     unsigned total = __reduce_add_sync(mask, adds);
     if ((threadIdx.x & 31) == (unsigned)(__ffs(mask) - 1) && total) atomicAdd(work, (unsigned long long)total);
 }
 
-constexpr int ACC_BLOCK_G1 = 512;   // lockstep block: 16 warps, one block per SM (<= 128 registers)
-
-// Chunks that a G1 accumulate block works on: all of its threads, or fewer, in
-// steps of a warp for each of the SM's four schedulers, when the chunks would
-// otherwise fill only some of the SMs.
-__device__ __forceinline__ uint32_t chunks_per_block(uint32_t M, uint32_t L) {
-    const uint32_t chunks = (uint32_t)(((uint64_t)M + L - 1) / L);
-    if (chunks >= MSM_SPREAD_THREADS) return ACC_BLOCK_G1;
-    constexpr uint32_t sms = MSM_SPREAD_THREADS / ACC_BLOCK_G1;
-    return ((chunks + sms - 1) / sms + 127) / 128 * 128;
-}
+// Small blocks: a thread's time varies with its bucket boundaries, and a small
+// MSM's chunks spread over the SMs.  Registers allow 16 warps an SM over G1
+// (four blocks at 128 registers) and 12 over G2 (three at 168).
+constexpr int ACC_BLOCK_G1 = 128;
 constexpr int ACC_BLOCK_G2 = 128;
-// G2 accumulate blocks resident per SM that the register budget must allow
-// (1: the compiler may take 255 registers, which leaves room for 2)
-#ifndef ACC_G2_MIN_BLOCKS
-#define ACC_G2_MIN_BLOCKS 1
-#endif
+constexpr int ACC_G1_BLOCKS = 4;
+constexpr int ACC_G2_BLOCKS = 3;
 
 // Multiprocessors of the current device (148 on a B200), cached per device.
 static uint32_t device_sms() {
@@ -548,8 +529,7 @@ static uint32_t device_sms() {
     return v;
 }
 
-// Threads in one wave of G1 accumulate blocks on the current device (one
-// block per SM), for chunk_len; 0 (no fitting) if the device cannot be read.
+// Threads in one wave of G1 accumulate blocks on the current device, for chunk_len; 0 (no fitting) if the device cannot be read.
 static uint32_t accumulate_wave() {
     static std::atomic<uint32_t> cache[64];
     int dev = 0;
@@ -558,13 +538,13 @@ static uint32_t accumulate_wave() {
     if (!w) {
         int sms = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return 0;
-        w = (uint32_t)sms * ACC_BLOCK_G1;
+        w = (uint32_t)sms * ACC_BLOCK_G1 * ACC_G1_BLOCKS;
         cache[dev].store(w, std::memory_order_relaxed);
     }
     return w;
 }
 
-__global__ void __launch_bounds__(ACC_BLOCK_G1, 1) k_accumulate_g1(const uint32_t* __restrict__ entries,
+__global__ void __launch_bounds__(ACC_BLOCK_G1, ACC_G1_BLOCKS) k_accumulate_g1(const uint32_t* __restrict__ entries,
                                                                    const uint32_t* __restrict__ offsets,
                                                                    const uint32_t* __restrict__ seg_base, uint32_t K,
                                                                    const uint32_t* __restrict__ d_M,
@@ -572,12 +552,10 @@ __global__ void __launch_bounds__(ACC_BLOCK_G1, 1) k_accumulate_g1(const uint32_
                                                                    const uint4* __restrict__ bases, uint32_t base_offset,
                                                                    uint32_t n_bases, uint4* __restrict__ partials,
                                                                    unsigned long long* __restrict__ work) {
-    const uint32_t M = *d_M, L = *d_L, per = chunks_per_block(M, L);
-    if ((size_t)blockIdx.x * per * L >= M) return;   // the whole block has no entries
-    accumulate_chunks<Fq, true>(entries, offsets, seg_base, K, M, L, bases, base_offset, n_bases, partials, work, per);
+    accumulate_chunks<Fq>(entries, offsets, seg_base, K, *d_M, *d_L, bases, base_offset, n_bases, partials, work);
 }
 
-__global__ void __launch_bounds__(ACC_BLOCK_G2, ACC_G2_MIN_BLOCKS) k_accumulate_g2(const uint32_t* __restrict__ entries,
+__global__ void __launch_bounds__(ACC_BLOCK_G2, ACC_G2_BLOCKS) k_accumulate_g2(const uint32_t* __restrict__ entries,
                                                                const uint32_t* __restrict__ offsets,
                                                                const uint32_t* __restrict__ seg_base, uint32_t K,
                                                                const uint32_t* __restrict__ d_M,
@@ -585,8 +563,7 @@ __global__ void __launch_bounds__(ACC_BLOCK_G2, ACC_G2_MIN_BLOCKS) k_accumulate_
                                                                const uint4* __restrict__ bases, uint32_t base_offset,
                                                                uint32_t n_bases, uint4* __restrict__ partials,
                                                                unsigned long long* __restrict__ work) {
-    accumulate_chunks<Fq2, false>(entries, offsets, seg_base, K, *d_M, *d_L, bases, base_offset, n_bases, partials,
-                                  work, blockDim.x);
+    accumulate_chunks<Fq2>(entries, offsets, seg_base, K, *d_M, *d_L, bases, base_offset, n_bases, partials, work);
 }
 
 __device__ __forceinline__ uint32_t n_partials(const uint32_t* offsets, uint32_t g, uint32_t L) {
@@ -959,7 +936,7 @@ __global__ void __launch_bounds__(256) k_scatter_multi(const MsmSourceDev* __res
     }
 }
 
-__global__ void __launch_bounds__(ACC_BLOCK_G1, 1) k_accumulate_multi_g1(const uint32_t* __restrict__ entries,
+__global__ void __launch_bounds__(ACC_BLOCK_G1, ACC_G1_BLOCKS) k_accumulate_multi_g1(const uint32_t* __restrict__ entries,
                                                                          const uint32_t* __restrict__ offsets,
                                                                          const uint32_t* __restrict__ seg_base,
                                                                          uint32_t K, const uint32_t* __restrict__ d_M,
@@ -967,13 +944,10 @@ __global__ void __launch_bounds__(ACC_BLOCK_G1, 1) k_accumulate_multi_g1(const u
                                                                          const MsmSegDev* __restrict__ segs,
                                                                          uint32_t nsegs, uint4* __restrict__ partials,
                                                                          unsigned long long* __restrict__ work) {
-    const uint32_t M = *d_M, L = *d_L, per = chunks_per_block(M, L);
-    if ((size_t)blockIdx.x * per * L >= M) return;   // the whole block has no entries
-    accumulate_chunks<Fq, true, true>(entries, offsets, seg_base, K, M, L, nullptr, 0, 0, partials, work, per, segs,
-                                      nsegs);
+    accumulate_chunks<Fq, true>(entries, offsets, seg_base, K, *d_M, *d_L, nullptr, 0, 0, partials, work, segs, nsegs);
 }
 
-__global__ void __launch_bounds__(ACC_BLOCK_G2, ACC_G2_MIN_BLOCKS) k_accumulate_multi_g2(const uint32_t* __restrict__ entries,
+__global__ void __launch_bounds__(ACC_BLOCK_G2, ACC_G2_BLOCKS) k_accumulate_multi_g2(const uint32_t* __restrict__ entries,
                                                                      const uint32_t* __restrict__ offsets,
                                                                      const uint32_t* __restrict__ seg_base,
                                                                      uint32_t K, const uint32_t* __restrict__ d_M,
@@ -981,8 +955,7 @@ __global__ void __launch_bounds__(ACC_BLOCK_G2, ACC_G2_MIN_BLOCKS) k_accumulate_
                                                                      const MsmSegDev* __restrict__ segs,
                                                                      uint32_t nsegs, uint4* __restrict__ partials,
                                                                      unsigned long long* __restrict__ work) {
-    accumulate_chunks<Fq2, false, true>(entries, offsets, seg_base, K, *d_M, *d_L, nullptr, 0, 0, partials, work,
-                                        blockDim.x, segs, nsegs);
+    accumulate_chunks<Fq2, true>(entries, offsets, seg_base, K, *d_M, *d_L, nullptr, 0, 0, partials, work, segs, nsegs);
 }
 
 // The bucket reduction of one segment of a space (msm_reduce_plan with one set).
@@ -1489,13 +1462,6 @@ cudaError_t msm_sort_sets(MsmSort* sorts, const MsmLiveSets& sets, const void* d
     return cudaSuccess;
 }
 
-// Blocks of a G1 accumulate over up to `chunks` chunks: enough for whole blocks
-// of chunks, and for the spread ones (chunks_per_block), one per SM at most.
-static unsigned accumulate_blocks_g1(size_t chunks) {
-    const unsigned spread = std::min<unsigned>(MSM_SPREAD_THREADS / ACC_BLOCK_G1, blocks_for(chunks, 128));
-    return std::max(blocks_for(chunks, ACC_BLOCK_G1), spread);
-}
-
 // threads of a k_reduce_sets block: a group per point of a term (nb a power of
 // two), a warp at least
 template <class F>
@@ -1531,7 +1497,7 @@ static cudaError_t accumulate(const MsmSort& s, MsmAccum& acc, const void* d_bas
     {
         TimedLaunch tl(tag, st);
         if (std::is_same<F, g16d::Fq>::value)
-            k_accumulate_g1<<<accumulate_blocks_g1(chunks), ACC_BLOCK_G1, 0, st>>>(
+            k_accumulate_g1<<<blocks_for(chunks, ACC_BLOCK_G1), ACC_BLOCK_G1, 0, st>>>(
                 s.d_entries, s.d_offsets, s.d_seg_base, s.Ks, s.d_total, s.d_total + 3, (const uint4*)d_bases,
                 base_offset, n_bases, partials, acc.d_work);
         else
@@ -1779,7 +1745,7 @@ static cudaError_t space_accumulate(MsmSpace& sp, cudaStream_t st, size_t xyzz_b
     if (chunks) {
         TimedLaunch tl(tag, st);
         if (std::is_same<F, g16d::Fq>::value)
-            k_accumulate_multi_g1<<<accumulate_blocks_g1(chunks), ACC_BLOCK_G1, 0, st>>>(
+            k_accumulate_multi_g1<<<blocks_for(chunks, ACC_BLOCK_G1), ACC_BLOCK_G1, 0, st>>>(
                 s.d_entries, s.d_offsets, s.d_seg_base, s.K, s.d_total, s.d_total + 3, (const MsmSegDev*)sp.d_segdev,
                 nsegs, partials, a.d_work);
         else
