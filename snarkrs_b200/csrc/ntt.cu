@@ -11,17 +11,37 @@ struct Vec3 {
     uint4* p[3];
 };
 
-__device__ __forceinline__ Fr ld_s(const uint4* sm, uint32_t e) {
-    uint4 a = sm[2 * e], b = sm[2 * e + 1];
-    Fr r;
-    r.v[0] = a.x; r.v[1] = a.y; r.v[2] = a.z; r.v[3] = a.w;
-    r.v[4] = b.x; r.v[5] = b.y; r.v[6] = b.z; r.v[7] = b.w;
-    return r;
-}
-__device__ __forceinline__ void st_s(uint4* sm, uint32_t e, const Fr& x) {
-    sm[2 * e] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
-    sm[2 * e + 1] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
-}
+// A tile in shared memory: the elements' low 16 bytes, then their high ones, so
+// that consecutive elements are consecutive 128-bit words, at a slot permuted
+// within 32 (slot bits 1, and 0 and 2, flipped by index bits 3 and 4): the 8
+// lanes that one 128-bit access serves then fall on different banks for the
+// element strides of every pair of stages.
+struct Tile {
+    uint4* lo;
+    uint4* hi;
+    __device__ __forceinline__ Tile(uint4* sm, uint32_t elems) : lo(sm), hi(sm + elems) {}
+    __device__ __forceinline__ static uint32_t slot(uint32_t e) {
+        return e ^ (((e >> 3) & 1u) << 1) ^ (((e >> 4) & 1u) * 5u);
+    }
+    __device__ __forceinline__ Fr ld(uint32_t e) const {
+        const uint32_t i = slot(e);
+        const uint4 a = lo[i], b = hi[i];
+        Fr r;
+        r.v[0] = a.x; r.v[1] = a.y; r.v[2] = a.z; r.v[3] = a.w;
+        r.v[4] = b.x; r.v[5] = b.y; r.v[6] = b.z; r.v[7] = b.w;
+        return r;
+    }
+    __device__ __forceinline__ void st(uint32_t e, const Fr& x) const {
+        const uint32_t i = slot(e);
+        lo[i] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
+        hi[i] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
+    }
+    __device__ __forceinline__ void fill(uint32_t e, const uint4* g, size_t gi) const {
+        const uint32_t i = slot(e);
+        lo[i] = g[2 * gi];
+        hi[i] = g[2 * gi + 1];
+    }
+};
 __device__ __forceinline__ Fr ld_g(const uint4* g, size_t i) {
     uint4 a = __ldg(g + 2 * i), b = __ldg(g + 2 * i + 1);
     Fr r;
@@ -41,37 +61,101 @@ __device__ __forceinline__ void st_g(uint4* g, size_t i, const Fr& x) {
     g[2 * i + 1] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
 }
 
+// A butterfly with twiddle tw[i] (i = 0: one).
+template <bool DIF>
+__device__ __forceinline__ void butterfly(Fr& a, Fr& b, const uint4* __restrict__ tw, size_t i) {
+    if (DIF) {
+        const Fr d = sub(a, b);
+        a = add(a, b);
+        b = i ? mul(d, ld_g(tw, i)) : d;
+    } else {
+        const Fr t = i ? mul(b, ld_g(tw, i)) : b;
+        b = sub(a, t);
+        a = add(a, t);
+    }
+}
+
 // One radix-2 stage on a shared-memory tile.  The tile holds elements
-// i = hi*2^(s_lo+k) + mid*2^s_lo + (lo0 + l) at smem slot mid*L + l; stage
+// i = hi*2^(s_lo+k) + mid*2^s_lo + (lo0 + l) at index mid*L + l; stage
 // s = s_lo + j pairs mid values differing in bit j.  The butterfly's
 // position inside its 2^(s+1) block is (mid mod 2^j)*2^s_lo + lo0 + l and
 // its twiddle omega_{2^(s+1)}^pos = tw[pos << (log_n - s - 1)].
 template <bool DIF>
-__device__ __forceinline__ void run_stage(uint4* sm, uint32_t j, uint32_t s_lo, uint32_t log_L, uint32_t lo0,
-                                          uint32_t log_n, uint32_t half_tile, const uint4* __restrict__ tw) {
-    const uint32_t L = 1u << log_L;
-    const uint32_t s = s_lo + j;
-    const uint32_t jmask = (1u << j) - 1u;
-    for (uint32_t q = threadIdx.x; q < half_tile; q += blockDim.x) {
-        uint32_t l = q & (L - 1u);
-        uint32_t mq = q >> log_L;
-        uint32_t mid_a = ((mq >> j) << (j + 1)) | (mq & jmask);
-        uint32_t ea = (mid_a << log_L) | l;
-        uint32_t eb = ea + (1u << (j + log_L));
-        uint32_t pos = ((mid_a & jmask) << s_lo) | (lo0 + l);
-        Fr a = ld_s(sm, ea), b = ld_s(sm, eb);
-        if (DIF) {
-            Fr d = sub(a, b);
-            a = add(a, b);
-            b = pos ? mul(d, ld_g(tw, (size_t)pos << (log_n - s - 1))) : d;
-        } else {
-            Fr t = pos ? mul(b, ld_g(tw, (size_t)pos << (log_n - s - 1))) : b;
-            b = sub(a, t);
-            a = add(a, t);
-        }
-        st_s(sm, ea, a);
-        st_s(sm, eb, b);
+__device__ __forceinline__ void run_stage(const Tile& t, uint32_t j, uint32_t s_lo, uint32_t log_L, uint32_t lo0,
+                                          uint32_t log_n, uint32_t tile, const uint4* __restrict__ tw) {
+    const uint32_t L = 1u << log_L, s = s_lo + j, jmask = (1u << j) - 1u;
+    for (uint32_t q = threadIdx.x; q < tile / 2; q += blockDim.x) {
+        const uint32_t l = q & (L - 1u), mq = q >> log_L;
+        const uint32_t mid = ((mq >> j) << (j + 1)) | (mq & jmask);
+        const uint32_t ea = (mid << log_L) | l, eb = ea + (1u << (j + log_L));
+        const uint32_t pos = ((mid & jmask) << s_lo) | (lo0 + l);
+        Fr a = t.ld(ea), b = t.ld(eb);
+        butterfly<DIF>(a, b, tw, (size_t)pos << (log_n - s - 1));
+        t.st(ea, a);
+        t.st(eb, b);
     }
+}
+
+// Stages j and j + 1 together, four elements in registers: half the trips
+// through shared memory and half the barriers of two single stages, and two
+// independent products at each step (intt_coset_ntt 2^20 433 us against 472 in
+// single stages, 2^22 1739 against 1859, each at its best tiling).  Bound by
+// the issue of wide multiply-adds: 55 G products/s at 2^22 of the 66.5 that a
+// bare product loop reaches.  80 registers (three blocks of 256 an SM).  With pos as above, stage j's two
+// butterflies share a twiddle; stage j + 1's sit at pos and pos + 2^(s_lo + j)
+// of their 2^(s+2) block.
+template <bool DIF>
+__device__ __forceinline__ void run_two_stages(const Tile& t, uint32_t j, uint32_t s_lo, uint32_t log_L, uint32_t lo0,
+                                               uint32_t log_n, uint32_t tile, const uint4* __restrict__ tw) {
+    const uint32_t L = 1u << log_L, s = s_lo + j, jmask = (1u << j) - 1u, step = 1u << (j + log_L);
+    for (uint32_t q = threadIdx.x; q < tile / 4; q += blockDim.x) {
+        const uint32_t l = q & (L - 1u), mq = q >> log_L;
+        const uint32_t mid = ((mq >> j) << (j + 2)) | (mq & jmask);
+        const uint32_t e = (mid << log_L) | l;
+        const uint32_t pos = ((mid & jmask) << s_lo) | (lo0 + l);
+        const size_t w0 = (size_t)pos << (log_n - s - 1), w1 = (size_t)pos << (log_n - s - 2),
+                     w2 = ((size_t)pos + ((size_t)1 << s)) << (log_n - s - 2);
+        Fr a = t.ld(e), b = t.ld(e + step), c = t.ld(e + 2 * step), d = t.ld(e + 3 * step);
+        if (DIF) {
+            butterfly<true>(a, c, tw, w1);
+            butterfly<true>(b, d, tw, w2);
+            butterfly<true>(a, b, tw, w0);
+            butterfly<true>(c, d, tw, w0);
+        } else {
+            butterfly<false>(a, b, tw, w0);
+            butterfly<false>(c, d, tw, w0);
+            butterfly<false>(a, c, tw, w1);
+            butterfly<false>(b, d, tw, w2);
+        }
+        t.st(e, a);
+        t.st(e + step, b);
+        t.st(e + 2 * step, c);
+        t.st(e + 3 * step, d);
+    }
+}
+
+// Stages [0, k) of a tile, from the top down (DIF) or the bottom up (DIT), two
+// at a time with an odd one out at the top; or single stages where the block
+// has a thread per butterfly (tile_threads).
+
+template <bool DIF>
+__device__ __forceinline__ void run_stages(const Tile& t, uint32_t k, uint32_t s_lo, uint32_t log_L, uint32_t lo0,
+                                           uint32_t log_n, const uint4* __restrict__ tw) {
+    const uint32_t tile = (1u << k) << log_L, pairs = 2 * blockDim.x >= tile ? 0 : k / 2;
+    if (DIF)
+        for (uint32_t j = k; j-- > 2 * pairs;) {
+            run_stage<true>(t, j, s_lo, log_L, lo0, log_n, tile, tw);
+            __syncthreads();
+        }
+    for (uint32_t i = 0; i < pairs; i++) {
+        run_two_stages<DIF>(t, DIF ? 2 * (pairs - 1 - i) : 2 * i, s_lo, log_L, lo0, log_n, tile, tw);
+        __syncthreads();
+    }
+    if (!DIF)
+        for (uint32_t j = 2 * pairs; j < k; j++) {
+            run_stage<false>(t, j, s_lo, log_L, lo0, log_n, tile, tw);
+            __syncthreads();
+        }
 }
 
 // Stages [s_lo, s_lo + k) of 2^log_n, one tile of (2^k)*L elements per block
@@ -84,27 +168,23 @@ __device__ __forceinline__ void ntt_pass_tile(uint4* sm, uint4* data, uint32_t b
                                               const uint4* __restrict__ join_b, uint4* __restrict__ join_out) {
     const uint32_t L = 1u << log_L;
     const uint32_t tile = (1u << k) << log_L;
+    const Tile t(sm, tile);
     const uint32_t bph = s_lo - log_L;
     const size_t hi = bx >> bph;
     const uint32_t lo0 = (bx & ((1u << bph) - 1u)) << log_L;
     for (uint32_t e = threadIdx.x; e < tile; e += blockDim.x) {
         uint32_t mid = e >> log_L, l = e & (L - 1u);
         size_t gi = (hi << (s_lo + k)) | ((size_t)mid << s_lo) | (lo0 + l);
-        sm[2 * e] = data[2 * gi];
-        sm[2 * e + 1] = data[2 * gi + 1];
+        t.fill(e, data, gi);
     }
     __syncthreads();
-    for (uint32_t jj = 0; jj < k; jj++) {
-        uint32_t j = DIF ? k - 1 - jj : jj;
-        run_stage<DIF>(sm, j, s_lo, log_L, lo0, log_n, tile / 2, tw);
-        __syncthreads();
-    }
+    run_stages<DIF>(t, k, s_lo, log_L, lo0, log_n, tw);
     Fr sc;
     if (scale) sc = ld_g(scale, 0);
     for (uint32_t e = threadIdx.x; e < tile; e += blockDim.x) {
         uint32_t mid = e >> log_L, l = e & (L - 1u);
         size_t gi = (hi << (s_lo + k)) | ((size_t)mid << s_lo) | (lo0 + l);
-        Fr x = ld_s(sm, e);
+        Fr x = t.ld(e);
         if (scale) x = mul(x, sc);
         if (join_out) {
             Fr h = sub(mul(ld_rw(join_a, gi), ld_rw(join_b, gi)), x);
@@ -117,7 +197,7 @@ __device__ __forceinline__ void ntt_pass_tile(uint4* sm, uint4* data, uint32_t b
 
 // blockIdx.y selects the vector
 template <bool DIF>
-__global__ void __launch_bounds__(256) k_ntt_pass(Vec3 vecs, uint32_t log_n, uint32_t s_lo, uint32_t k,
+__global__ void __launch_bounds__(256, 3) k_ntt_pass(Vec3 vecs, uint32_t log_n, uint32_t s_lo, uint32_t k,
                                                   uint32_t log_L, const uint4* __restrict__ tw,
                                                   const uint4* __restrict__ scale, const uint4* __restrict__ join_a,
                                                   const uint4* __restrict__ join_b, uint4* __restrict__ join_out) {
@@ -135,24 +215,16 @@ __device__ __forceinline__ void ntt_mid_tile(uint4* sm, uint4* data, uint32_t bx
                                              const uint4* __restrict__ coset, const uint4* __restrict__ join_a,
                                              const uint4* __restrict__ join_b, uint4* __restrict__ join_out) {
     const uint32_t tile = 1u << k;
+    const Tile t(sm, tile);
     const size_t base = (size_t)bx << k;
-    for (uint32_t e = threadIdx.x; e < tile; e += blockDim.x) {
-        sm[2 * e] = data[2 * (base + e)];
-        sm[2 * e + 1] = data[2 * (base + e) + 1];
-    }
+    for (uint32_t e = threadIdx.x; e < tile; e += blockDim.x) t.fill(e, data, base + e);
     __syncthreads();
-    for (int j = (int)k - 1; j >= 0; j--) {
-        run_stage<true>(sm, (uint32_t)j, 0, 0, 0, log_n, tile / 2, tw_inv);
-        __syncthreads();
-    }
-    for (uint32_t e = threadIdx.x; e < tile; e += blockDim.x) st_s(sm, e, mul(ld_s(sm, e), ld_g(coset, base + e)));
+    run_stages<true>(t, k, 0, 0, 0, log_n, tw_inv);
+    for (uint32_t e = threadIdx.x; e < tile; e += blockDim.x) t.st(e, mul(t.ld(e), ld_g(coset, base + e)));
     __syncthreads();
-    for (uint32_t j = 0; j < k; j++) {
-        run_stage<false>(sm, j, 0, 0, 0, log_n, tile / 2, tw);
-        __syncthreads();
-    }
+    run_stages<false>(t, k, 0, 0, 0, log_n, tw);
     for (uint32_t e = threadIdx.x; e < tile; e += blockDim.x) {
-        Fr x = ld_s(sm, e);
+        Fr x = t.ld(e);
         if (join_out) {
             st_g(join_out, base + e, sub(mul(ld_rw(join_a, base + e), ld_rw(join_b, base + e)), x));
         } else {
@@ -165,25 +237,20 @@ __device__ __forceinline__ void ntt_mid_tile(uint4* sm, uint4* data, uint32_t bx
 // each position p multiplied by table[p] and stored: the last step of an
 // inverse transform to bit-reversed order with a per-position scale (gnark's
 // H coefficients: table = shift^-bitrev(p) / n).
-__global__ void __launch_bounds__(256) k_ntt_dif_scale(uint4* data, uint32_t log_n, uint32_t k,
+__global__ void __launch_bounds__(256, 3) k_ntt_dif_scale(uint4* data, uint32_t log_n, uint32_t k,
                                                        const uint4* __restrict__ tw_inv,
                                                        const uint4* __restrict__ table) {
     extern __shared__ uint4 sm[];
     const uint32_t tile = 1u << k;
+    const Tile t(sm, tile);
     const size_t base = (size_t)blockIdx.x << k;
-    for (uint32_t e = threadIdx.x; e < tile; e += blockDim.x) {
-        sm[2 * e] = data[2 * (base + e)];
-        sm[2 * e + 1] = data[2 * (base + e) + 1];
-    }
+    for (uint32_t e = threadIdx.x; e < tile; e += blockDim.x) t.fill(e, data, base + e);
     __syncthreads();
-    for (int j = (int)k - 1; j >= 0; j--) {
-        run_stage<true>(sm, (uint32_t)j, 0, 0, 0, log_n, tile / 2, tw_inv);
-        __syncthreads();
-    }
-    for (uint32_t e = threadIdx.x; e < tile; e += blockDim.x) st_g(data, base + e, mul(ld_s(sm, e), ld_g(table, base + e)));
+    run_stages<true>(t, k, 0, 0, 0, log_n, tw_inv);
+    for (uint32_t e = threadIdx.x; e < tile; e += blockDim.x) st_g(data, base + e, mul(t.ld(e), ld_g(table, base + e)));
 }
 
-__global__ void __launch_bounds__(256) k_ntt_mid(Vec3 vecs, uint32_t log_n, uint32_t k, const uint4* __restrict__ tw,
+__global__ void __launch_bounds__(256, 3) k_ntt_mid(Vec3 vecs, uint32_t log_n, uint32_t k, const uint4* __restrict__ tw,
                                                  const uint4* __restrict__ tw_inv, const uint4* __restrict__ coset,
                                                  const uint4* __restrict__ join_a, const uint4* __restrict__ join_b,
                                                  uint4* __restrict__ join_out) {
@@ -216,14 +283,14 @@ __device__ __forceinline__ uint32_t job_of(const NttJob* __restrict__ jobs, uint
 }
 
 template <bool DIF>
-__global__ void __launch_bounds__(256) k_ntt_pass_multi(const NttJob* __restrict__ jobs, uint32_t njobs) {
+__global__ void __launch_bounds__(256, 3) k_ntt_pass_multi(const NttJob* __restrict__ jobs, uint32_t njobs) {
     extern __shared__ uint4 sm[];
     const NttJob& j = jobs[job_of(jobs, njobs, blockIdx.x)];
     ntt_pass_tile<DIF>(sm, j.data, blockIdx.x - j.block_start, j.log_n, j.s_lo, j.k, j.log_L, j.tw, nullptr, j.join_a,
                        j.join_b, j.join_out);
 }
 
-__global__ void __launch_bounds__(256) k_ntt_mid_multi(const NttJob* __restrict__ jobs, uint32_t njobs) {
+__global__ void __launch_bounds__(256, 3) k_ntt_mid_multi(const NttJob* __restrict__ jobs, uint32_t njobs) {
     extern __shared__ uint4 sm[];
     const NttJob& j = jobs[job_of(jobs, njobs, blockIdx.x)];
     ntt_mid_tile(sm, j.data, blockIdx.x - j.block_start, j.log_n, j.k, j.tw, j.tw_inv, j.coset, j.join_a, j.join_b,
@@ -339,6 +406,7 @@ cudaError_t ntt_tables(NttTables& t, int log_n, cudaStream_t st) {
     G16_CUDA(cudaMemcpyAsync((uint8_t*)t.d_coset + n * 32, ninv.x.v, 32, cudaMemcpyHostToDevice, st));
     G16_CUDA(cudaGetLastError());
     G16_CUDA(cudaStreamSynchronize(st));
+    t.tiling = ntt_default_tiling((uint32_t)log_n);
     t.log_n = log_n;
     return cudaSuccess;
 }
@@ -363,12 +431,21 @@ static void set_attrs() {
     attrs_done = true;
 }
 
+// Threads of a tile's block: one per four elements, a warp at least.  A lone
+// transform's small tiles get one per butterfly instead: it is their latency
+// that counts, and two warps a scheduler hide more of it than one with two
+// products at a time (2^8 25 against 29 us).
+static unsigned tile_threads(uint32_t tile, bool alone) {
+    const uint32_t t = alone && tile <= 256 ? tile / 2 : tile / 4;
+    return t < 32 ? 32 : t < 256 ? t : 256;
+}
+
 static cudaError_t launch_pass(bool dif, Vec3 v, int nv, uint32_t log_n, const Pass& p, const void* tw,
                                const void* scale, const void* ja, const void* jb, void* jo, cudaStream_t st) {
     uint32_t tile = (1u << p.k) << p.log_L;
     size_t n = (size_t)1 << log_n;
     dim3 grid((unsigned)(n / tile), nv);
-    unsigned threads = tile / 2 < 256 ? tile / 2 : 256;
+    const unsigned threads = tile_threads(tile, true);
     size_t smem = (size_t)tile * 32;
     const char* name = dif ? "ntt_pass_dif" : "ntt_pass_dit";
     // work: one Fr product per butterfly, plus the scale / join epilogue;
@@ -394,7 +471,7 @@ static cudaError_t launch_mid(Vec3 v, int nv, const NttTables& t, const void* ja
     uint32_t tile = 1u << k0;
     size_t n = (size_t)1 << log_n;
     dim3 grid((unsigned)(n / tile), nv);
-    unsigned threads = tile / 2 < 256 ? tile / 2 : 256;
+    const unsigned threads = tile_threads(tile, true);
     timer().add_units("ntt_mid_fused", (double)nv * ((double)n * k0 + n) + (jo ? (double)n : 0.0));
     timer().add_bytes("ntt_mid_fused", 64.0 * nv * n + (jo ? 64.0 * n : 0.0));
     TimedLaunch tl("ntt_mid_fused", st);
@@ -493,7 +570,7 @@ cudaError_t ntt_to_gnark_coefficients(const NttTables& t, void* h, cudaStream_t 
         G16_CUDA(launch_pass(true, v, 1, log_n, outer[i], t.d_tw_inv, nullptr, nullptr, nullptr, nullptr, st));
     const uint32_t tile = 1u << k0;
     const size_t n = (size_t)1 << log_n;
-    const unsigned threads = tile / 2 < 256 ? tile / 2 : 256;
+    const unsigned threads = tile_threads(tile, true);
     timer().add_units("ntt_pass_dif", (double)(n / 2) * k0 + (double)n);
     timer().add_bytes("ntt_pass_dif", 64.0 * n);
     TimedLaunch tl("ntt_pass_dif", st);
@@ -560,11 +637,13 @@ cudaError_t ntt_batch_setup(NttBatch& nb, const std::vector<NttBatchItem>& items
         ph.njobs = (uint32_t)jobs.size();
         uint32_t blocks = 0;
         size_t smem = 0;
+        ph.threads = 32;
         for (auto& j : jobs) {
             j.block_start = blocks;
             const uint32_t tile = kind == 2 ? (1u << j.k) : ((1u << j.k) << j.log_L);
             blocks += (uint32_t)(((size_t)1 << j.log_n) / tile);
             smem = std::max(smem, (size_t)tile * 32);
+            ph.threads = std::max(ph.threads, tile_threads(tile, false));
             ph.products += kind == 2 ? ((double)((size_t)1 << j.log_n) * (j.k + 1)) : ((double)((size_t)1 << j.log_n) / 2 * j.k);
             ph.bytes += 64.0 * (double)((size_t)1 << j.log_n) * (j.join_out ? 2 : 1);
         }
@@ -630,9 +709,9 @@ cudaError_t ntt_batch_run(const NttBatch& nb, cudaStream_t st) {
         timer().add_units(name, ph.products);
         timer().add_bytes(name, ph.bytes);
         TimedLaunch tl(name, st);
-        if (ph.kind == 0) k_ntt_pass_multi<true><<<ph.blocks, 256, ph.smem, st>>>(jobs, ph.njobs);
-        else if (ph.kind == 1) k_ntt_pass_multi<false><<<ph.blocks, 256, ph.smem, st>>>(jobs, ph.njobs);
-        else k_ntt_mid_multi<<<ph.blocks, 256, ph.smem, st>>>(jobs, ph.njobs);
+        if (ph.kind == 0) k_ntt_pass_multi<true><<<ph.blocks, ph.threads, ph.smem, st>>>(jobs, ph.njobs);
+        else if (ph.kind == 1) k_ntt_pass_multi<false><<<ph.blocks, ph.threads, ph.smem, st>>>(jobs, ph.njobs);
+        else k_ntt_mid_multi<<<ph.blocks, ph.threads, ph.smem, st>>>(jobs, ph.njobs);
         G16_CUDA(cudaGetLastError());
     }
     return cudaSuccess;

@@ -28,14 +28,29 @@ namespace g16 {
 // columns per tile row).  The values are the same for every tiling; only the
 // number of passes over HBM and the shared-memory footprint change.
 struct NttTiling {
-    uint32_t tile_log = 11;      // 2048 elements, 64 KiB of shared memory
-    uint32_t outer_log_l = 2;    // 4 columns = 128-byte rows
+    uint32_t tile_log = 9;       // 512 elements, 16 KiB of shared memory
+    uint32_t outer_log_l = 3;    // 8 columns = 256-byte rows
 };
 constexpr uint32_t NTT_MAX_TILE_LOG = 12;   // 128 KiB of shared memory
 
 // Is the tiling one the kernels accept?
 inline bool ntt_tiling_valid(const NttTiling& t) {
     return t.tile_log >= 2 && t.tile_log <= NTT_MAX_TILE_LOG && t.outer_log_l < t.tile_log && t.outer_log_l <= 4;
+}
+
+// The tiling a transform of 2^log_n starts with.  Small tiles: a block of 256
+// elements or so leaves its SM to others while it waits at a barrier, and a
+// small transform reaches more SMs.  Rows of 8 columns, or of 4 where the
+// stages left by the inner pass then fit one outer pass instead of two.
+// intt_coset_ntt by the inner tile, us (2^11 with rows of 4 was the one tiling
+// for every size): 2^12 40 (2^8) against 101, 2^16 63 (2^8) against 115, 2^18
+// 145 (2^9) against 153, 2^20 433 (2^9) against 502, 2^22 1739 (2^10) against
+// 1819; 2^9 at 2^22 takes 1856, 2^10 at 2^20 450.
+inline NttTiling ntt_default_tiling(uint32_t log_n) {
+    NttTiling t;
+    t.tile_log = log_n <= 17 ? 8 : log_n <= 21 ? 9 : 10;
+    t.outer_log_l = log_n <= 2 * t.tile_log - 2 ? 2 : 3;
+    return t;
 }
 
 // The passes of a transform of 2^log_n under a tiling (host arithmetic only, so
@@ -184,7 +199,7 @@ struct NttBatchItem {
 };
 struct NttPhase {
     int kind = 0;           // 0 inverse outer pass, 1 forward outer pass, 2 fused middle
-    uint32_t first = 0, njobs = 0, blocks = 0;
+    uint32_t first = 0, njobs = 0, blocks = 0, threads = 256;
     size_t smem = 0;
     double products = 0, bytes = 0;   // algorithmic work, for the kernel timer
 };
