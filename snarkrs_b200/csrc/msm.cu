@@ -1132,10 +1132,16 @@ void MsmAccum::release() {
 }
 
 int msm_shared_window_bits(size_t m) {
-    int best = 8;
+    // A bucket costs about six mixed additions over one shared set: two additions
+    // of the reduction, of four products on a group of lanes, and its share of
+    // the bucket sums.  Below 10 bits the buckets are so few that chunks run
+    // long and the small MSM loses its threads.  Witness widths of the default
+    // circuits against three additions a bucket: 2^15 constraints 15 -> 13 bits,
+    // prove 1139 -> 1034 us; 2^17 16 -> 15, 2301 -> 2254 us; 1.1M 17 either way.
+    int best = 10;
     double best_cost = 1e300;
-    for (int c = 8; c <= 22; c++) {
-        double cost = (double)m * msm_windows(c) + 3.0 * (double)(1u << (c - 1));
+    for (int c = 10; c <= 22; c++) {
+        double cost = (double)m * msm_windows(c) + 6.0 * (double)(1u << (c - 1));
         if (cost < best_cost) {
             best_cost = cost;
             best = c;
@@ -1211,13 +1217,14 @@ cudaError_t msm_window_table_g2(const void* d_in, size_t n, uint32_t skip, int c
 }
 
 int msm_window_bits(size_t m) {
-    // cost ~ windows * (m + 2 * buckets): bucket reduction runs fully parallel
-    // on the device, so buckets weigh less than the reference CPU model's 3
+    // cost ~ windows * (m + 3.75 * buckets), a bucket at about four mixed additions
+    // (measured: 2^16 points 637 us at 12 bits, 699 at 13 and 14; 2^18 1330 at 15,
+    // 1472 at 13, 1517 at 16; 2^20 3690 at 16, 3625 at 15, 3895 at 17)
     int best = 8;
     double best_cost = 1e300;
     for (int c = 8; c <= 18; c++) {
         double windows = (255 + c - 1) / c;
-        double cost = windows * ((double)m + 2.0 * (double)(1u << (c - 1)));
+        double cost = windows * ((double)m + 3.75 * (double)(1u << (c - 1)));
         if (cost < best_cost) {
             best_cost = cost;
             best = c;
