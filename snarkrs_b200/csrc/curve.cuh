@@ -3,8 +3,9 @@
 // Buckets and running sums use XYZZ coordinates (x = X/ZZ, y = Y/ZZZ,
 // ZZ^3 = ZZZ^2), the representation the reference's MSMs accumulate in
 // (crates/msm/src/xyzz.rs; crates/cuda/src/kernels/bn254_curve.cuh:486-600).
-// Formulas are the Explicit-Formulas Database ones for a = 0:
-// madd-2008-s (8M + 2S), add-2008-s (12M + 2S), mdbl-2008-s-1 and
+// Formulas are the Explicit-Formulas Database ones for a = 0 (add-2008-s is in
+// lanes.cuh):
+// madd-2008-s (8M + 2S), mdbl-2008-s-1 and
 // dbl-2008-s-1.  ZZ = 0 is the identity.  The three exceptional cases of an
 // incomplete addition (identity operand, P + P, P + (-P)) are handled
 // explicitly: they are rare but reachable (duplicate bases, a bucket that
@@ -87,10 +88,6 @@ template <class F>
 __device__ __noinline__ Xyzz<F> xyzz_dbl_affine_ool(F x, F y) {
     return xyzz_dbl_affine<F, false>(x, y);
 }
-template <class F>
-__device__ __noinline__ Xyzz<F> xyzz_dbl_ool(Xyzz<F> p) {
-    return xyzz_dbl<F, false>(p);
-}
 
 // p + (x2, y2) for a finite affine point (madd-2008-s)
 template <class F, bool INL = true>
@@ -131,30 +128,6 @@ __device__ __forceinline__ Xyzz<F> xyzz_add_affine(const Xyzz<F>& p, const F& x2
         r.y = sub(t, ypp);
         r.zz = fmul<INL>(p.zz, pp);
     }
-    return r;
-}
-
-// p + q (add-2008-s)
-template <class F, bool INL = true>
-__device__ __forceinline__ Xyzz<F> xyzz_add(const Xyzz<F>& p, const Xyzz<F>& q) {
-    if (p.is_inf()) return q;
-    if (q.is_inf()) return p;
-    F u1, u2, s1, s2, zz12, zzz12;
-    fmul3<INL>(p.x, q.zz, q.x, p.zz, p.zz, q.zz, u1, u2, zz12);
-    fmul3<INL>(p.y, q.zzz, q.y, p.zzz, p.zzz, q.zzz, s1, s2, zzz12);
-    F pp_ = sub(u2, u1);
-    F rr = sub(s2, s1);
-    if (pp_.is_zero()) {
-        if (rr.is_zero()) return xyzz_dbl_ool<F>(p);   // rare: keep it out of the hot code
-        return Xyzz<F>::identity();
-    }
-    F pp, rr2, ppp, qq, t, sppp;
-    fmul2<INL>(pp_, pp_, rr, rr, pp, rr2);
-    Xyzz<F> r;
-    fmul3<INL>(pp_, pp, u1, pp, zz12, pp, ppp, qq, r.zz);
-    r.x = sub(sub(rr2, ppp), dbl(qq));
-    fmul3<INL>(rr, sub(qq, r.x), s1, ppp, zzz12, ppp, t, sppp, r.zzz);
-    r.y = sub(t, sppp);
     return r;
 }
 

@@ -135,8 +135,7 @@ __global__ void __launch_bounds__(256) k_scatter(const uint4* __restrict__ scala
 // Set j keeps scalar i when rank[j][i] != MSM_DEAD; its entries name row
 // rank[j][i] of the set's own window-shifted table: w * rows[j] + rank[j][i].
 // The digits are computed once and sorted into every set the scalar is live
-// in, so a base at infinity never becomes an entry (a lockstep step of the
-// accumulate that adds nothing).
+// in, so a base at infinity never becomes an entry.
 // With per-window bucket sets instead (plain bases, a compact key) window w's
 // digit d goes to bucket w B + |d| - 1 and its entry is rank[j][i] itself:
 // key_stride = B and rows = 0.

@@ -49,13 +49,11 @@ namespace g16 {
 //   set sum = T + seg (sum_j 2^j G_j + 2^lb sum_i 2^i Gb_i).
 // seg grows (up to 32) until the pieces over all sets number at most the
 // target.  Fewer, longer pieces keep the reduction's footprint small where it
-// runs beside other MSMs' accumulations, whose 512-thread blocks need a whole
-// SM: the prover's window-shifted MSMs (one bucket set) aim at 8192 pieces,
-// measured best for the 2^21-constraint prove (45.7 proofs/s against 44.1
-// with 32768) and equal at 2^17.  A standalone MSM (one set per window) has
-// the GPU to itself and aims at 32768, shortening the chains; so does the
-// prover's H MSM (MsmSort::reduce_pieces), whose reduction runs last, when the
-// witness MSMs' accumulations are mostly done.
+// runs beside other MSMs' accumulations: the prover's window-shifted MSMs (one
+// bucket set) aim at 8192 pieces, 512 threads an SM over G1.  A standalone MSM
+// (one set per window) has the GPU to itself and aims at 32768, shortening the
+// chains; so does the prover's H MSM (MsmSort::reduce_pieces), whose reduction
+// runs last, when the witness MSMs' accumulations are mostly done.
 constexpr uint64_t MSM_REDUCE_PIECES = 8192;
 constexpr uint64_t MSM_REDUCE_PIECES_ALONE = 32768;
 constexpr uint32_t MSM_REDUCE_MAX_SEG = 32;

@@ -343,12 +343,6 @@ __global__ void k_bitrev(uint4* a, uint32_t log_n, uint64_t n) {
     }
 }
 
-__global__ void k_join(const uint4* a, const uint4* b, const uint4* c, uint4* h, uint64_t n) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    st_g(h, i, sub(mul(ld_rw(a, i), ld_rw(b, i)), ld_rw(c, i)));
-}
-
 }  // namespace g16d
 
 namespace g16 {

@@ -1986,8 +1986,8 @@ int g16_autotune(g16_circuit* c, const uint8_t* w, size_t n, int concurrency, g1
     {
         NttTiling best = c->ntt.tiling;
         double best_t = -1;
-        for (uint32_t tl : {10u, 11u, 12u})
-            for (uint32_t ll : {1u, 2u, 3u}) {
+        for (uint32_t tl : {8u, 9u, 10u, 11u})
+            for (uint32_t ll : {2u, 3u}) {
                 if ((uint32_t)c->log_n <= 10 && !(tl == best.tile_log && ll == best.outer_log_l)) continue;
                 c->ntt.tiling = {tl, ll};
                 double t = together ? whole()
