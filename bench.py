@@ -41,18 +41,21 @@ R_MOD = 218882428718392752222464057452572750885483644004160343436982041865758084
 N_CONSTRAINTS = 1_100_000
 N_INPUTS, N_PUBLIC = 256, 16
 CIRCUIT_SEED, TOXIC_SEED = 21, 0x5EED
-FQ_MUL_IMAD = 264            # 8x32-bit CIOS Montgomery product: 32-bit multiply-adds
-FQ_SQR_IMAD = 208            # separated squaring: 36 limb products + 8 x 17 for the reduction
-FQ2_MUL_IMAD = 3 * 128 + 2 * 136   # three 8x8-limb products, two Montgomery reductions
-FQ_MUL_SUB_IMAD = 2 * 128 + 136    # a b - c d: two 8x8-limb products, one reduction
-# 32-bit multiply-adds per mixed addition (madd-2008-s, 8M + 2S): G1 squares with
-# the separated squaring and forms Y3 = R (Q - X3) - Y1 PPP with one reduction;
-# G2 runs all ten as Fq2 products with deferred reduction (656 IMAD each: its two
-# squares as products too, which measured faster than separate Fq2 squares)
+# Integer work in units of the peak probe's average multiply-add (g16_imad_peak: one mad.lo,
+# 64 a clock on an SM, to one mad.hi, 32 a clock): a 32x32+64-bit wide multiply-add, 32 a clock,
+# is 4/3 of it and a mad.lo 2/3.
+WIDE, LO = 4 / 3, 2 / 3
+FQ_MUL_IMAD = 128 * WIDE + 8 * LO             # 8x32-bit CIOS Montgomery product
+FQ_SQR_IMAD = (36 + 64) * WIDE + 8 * LO       # separated squaring, then the reduction
+FQ2_MUL_IMAD = (3 * 64 + 2 * 64) * WIDE + 16 * LO   # three 8x8-limb products, two reductions
+FQ2_SQR_IMAD = 2 * FQ_MUL_IMAD                # (a0 + a1)(a0 - a1) and a0 a1
+FQ_MUL_SUB_IMAD = (2 * 64 + 64) * WIDE + 8 * LO     # a b - c d: two products, one reduction
+# per mixed addition (madd-2008-s, 8M + 2S): G1 forms Y3 = R (Q - X3) - Y1 PPP with one reduction
 MADD_IMAD = {"msm_accumulate_g1": 6 * FQ_MUL_IMAD + 2 * FQ_SQR_IMAD + FQ_MUL_SUB_IMAD,
-             "msm_accumulate_g2": 10 * FQ2_MUL_IMAD}
-MADD_WORK = {"msm_accumulate_g1": "6 Fq products x 264 + 2 Fq squares x 208 + 1 product difference x 392 IMAD",
-             "msm_accumulate_g2": "10 Fq2 products x 656 IMAD"}
+             "msm_accumulate_g2": 8 * FQ2_MUL_IMAD + 2 * FQ2_SQR_IMAD}
+MADD_WORK = {"msm_accumulate_g1": "6 Fq products x 128 + 2 Fq squares x 100 + 1 product difference x 192 wide "
+                                  "multiply-adds",
+             "msm_accumulate_g2": "8 Fq2 products x 320 + 2 Fq2 squares x 256 wide multiply-adds"}
 
 
 # g16_ntt modes (CpuNtt, crates/ntt/src/lib.rs:415-584) by bench name
@@ -635,7 +638,7 @@ def reference_window_size(m):
 def msm_work_model(scalars, g2):
     """Algorithmic work of one MSM by the reference's model: m general (not 0 or 1) scalars,
     c = window_size(m), W = ceil(255/c), B = 2^(c-1); Fq products = 10 m W + 28 B W plus 10 per
-    scalar equal to 1, three times that in G2; 264 IMAD per Fq product."""
+    scalar equal to 1, three times that in G2; FQ_MUL_IMAD per Fq product."""
     import numpy as np
     v = np.frombuffer(scalars, dtype=np.uint64).reshape(-1, 4)
     high_zero = (v[:, 1] | v[:, 2] | v[:, 3]) == 0
