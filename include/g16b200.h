@@ -195,7 +195,7 @@ typedef struct {
     int msm_window_bits_witness;   /* c of the A, B1, L, B2 MSMs */
     int msm_window_bits_h;         /* c of the H MSM */
     uint64_t key_bytes;            /* device bytes of the prepared key */
-    uint64_t workspace_bytes;      /* device bytes of one proof in flight */
+    uint64_t workspace_bytes;      /* device bytes of one proof in flight, at least (more where there is room) */
 } g16_key_plan;
 /* The plan g16_prepare follows with free_bytes of device memory: window tables
  * when the key, its tables and one workspace fit; else the compact key when it

@@ -12,6 +12,7 @@ namespace g16d {
 
 using g16::MSM_DEAD;
 using g16::MSM_MAX_SETS;
+using g16::MSM_CHUNK;
 using g16::MSM_SPREAD_THREADS;
 using g16::MSM_MAX_TARGETS;
 
@@ -287,7 +288,7 @@ __device__ __forceinline__ uint32_t chunk_len(uint32_t M, uint32_t K, uint32_t L
 // one 0.83 -> 0.29 ms, of 1000 uniform points 0.20 -> 0.03 ms.
 __device__ __forceinline__ uint32_t min_chunk(uint32_t M, uint32_t floor) {
     const uint32_t spread = (M + MSM_SPREAD_THREADS - 1) / MSM_SPREAD_THREADS;
-    const uint32_t L = spread < 16 ? spread : 16;
+    const uint32_t L = spread < MSM_CHUNK ? spread : MSM_CHUNK;
     return L > floor ? L : floor;
 }
 
@@ -1320,9 +1321,9 @@ cudaError_t msm_sort(MsmSort& s, const void* d_scalars, size_t n, bool montgomer
         set_error("MSM of %zu points x %d windows exceeds the 2^31 entry-index limit", n, s.W);
         return cudaErrorInvalidValue;
     }
-    // the smallest chunk the accumulate may use (fixed scratch is sized for 16);
+    // the smallest chunk the accumulate may use (fixed scratch is sized for MSM_CHUNK);
     // the one it does use is chosen on the device from the entry count
-    s.chunk = s.fixed ? 16 : MSM_MIN_CHUNK;
+    s.chunk = s.fixed ? MSM_CHUNK : s.chunk_floor;
     const uint32_t kw = shared_windows ? 0u : s.B, ew = shared_windows ? (uint32_t)n : 0u;
     const uint32_t sink = constant_work ? s.K : NO_KEY;
     size_t nn = n ? n : 1;
@@ -1405,7 +1406,7 @@ cudaError_t msm_sort_sets(MsmSort* sorts, const MsmLiveSets& sets, const void* d
         s.constant_work = constant_work;
         s.Ks = s.K + (constant_work ? 1u : 0u);
         s.n = sets.rows[j];
-        s.chunk = MSM_MIN_CHUNK;
+        s.chunk = s.chunk_floor;
         if ((size_t)sets.rows[j] * (size_t)W >= 0x80000000ull || sets.rows[j] > n) {
             set_error("live set of %u rows x %d windows exceeds the 2^31 entry-index limit", sets.rows[j], W);
             return cudaErrorInvalidValue;
@@ -1639,7 +1640,7 @@ cudaError_t msm_batch_setup(MsmSources& so, MsmSpace* const* spaces, int nspaces
         s.K = s.Ks = sp.K;
         s.B = 0;
         s.shared = true;
-        s.chunk = MSM_MIN_CHUNK;
+        s.chunk = s.chunk_floor;
         s.n = sp.max_entries;   // accumulate sizes its partials by entries, W = 1 below
         s.W = 1;
         const size_t kk = (size_t)sp.K + 1;

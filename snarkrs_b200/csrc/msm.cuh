@@ -146,14 +146,16 @@ inline MsmSpaceReduceLayout msm_space_reduce_layout(const std::vector<uint32_t>&
     return L;
 }
 
-// Accumulate chunks (sorted entries per thread): 16 or more, or down to
-// MSM_MIN_CHUNK when 16 would leave SMs without their 512 threads (min_chunk in
-// msm.cu).  Buffers hold the most chunks any entry count up to the maximum can
-// give.
+// Accumulate chunks (sorted entries per thread): MSM_CHUNK or more, or down to
+// MSM_MIN_CHUNK when that would leave SMs without their 512 threads (min_chunk
+// in msm.cu).  Buffers hold the most chunks any entry count up to the maximum
+// can give: up to 58 MB more for a proof with the smaller floor, which a device
+// memory budget without room for it keeps off (MsmSort::chunk_floor).
+constexpr uint32_t MSM_CHUNK = 16;
 constexpr uint32_t MSM_MIN_CHUNK = 4;
 constexpr uint32_t MSM_SPREAD_THREADS = 148 * 512;
 constexpr size_t msm_max_chunks(size_t max_entries, uint32_t floor) {
-    const size_t whole = (max_entries + 15) / 16, least = (max_entries + floor - 1) / floor;
+    const size_t whole = (max_entries + MSM_CHUNK - 1) / MSM_CHUNK, least = (max_entries + floor - 1) / floor;
     const size_t spread = least < MSM_SPREAD_THREADS ? least : MSM_SPREAD_THREADS;
     return whole > spread ? whole : spread;
 }
@@ -168,7 +170,8 @@ struct MsmSort {
     bool constant_work = false;   // zero digits are sorted into the sink bucket K
     uint64_t reduce_pieces = 0;   // bucket-reduction piece target; 0: msm_reduce_pieces(shared)
     size_t n = 0;          // scalars sorted
-    uint32_t chunk = 16;   // smallest accumulate chunk
+    uint32_t chunk_floor = MSM_MIN_CHUNK;   // MSM_CHUNK where scratch has to stay small
+    uint32_t chunk = MSM_CHUNK;             // smallest accumulate chunk of the last sort
     // device buffers (capacities in elements)
     uint32_t* d_scalars_std = nullptr;  size_t cap_scalars = 0;   // 8 u32 per scalar
     uint32_t* d_counts = nullptr;       size_t cap_k = 0;         // K + 1

@@ -261,14 +261,15 @@ cudaError_t circuit_alloc(g16_circuit* c, void** p, size_t bytes) {
 // Device bytes of one workspace: witness, A|B|C, H, and the MSM scratch
 // (sorted entries, partial sums, bucket sums) at window bits c_w and c_h, for
 // live sets of ra (A), rb (B1, B2) and rl (L) wires; tables: one bucket set
-// per MSM (window tables), else one per window (compact key).
+// per MSM (window tables), else one per window (compact key); chunk_floor: the
+// MSMs' smallest accumulate chunk.
 uint64_t workspace_estimate(uint64_t nv, uint64_t n, int c_w, int c_h, uint64_t ra, uint64_t rb, uint64_t rl,
-                            bool tables) {
+                            bool tables, uint32_t chunk_floor) {
     const uint64_t Ww = (uint64_t)msm_windows(c_w), Wh = (uint64_t)msm_windows(c_h);
     const uint64_t Kw = (1ull << (c_w - 1)) * (tables ? 1 : Ww), Kh = (1ull << (c_h - 1)) * (tables ? 1 : Wh);
     uint64_t b = nv * 32 + n * 32 * 4;
     b += nv * 32 + (ra + rb + rl) * Ww * 4 + 3 * 24 * (Kw + 1) + n * 32 + n * Wh * 4 + 24 * (Kh + 1);
-    auto chunks = [](uint64_t entries) { return (uint64_t)msm_max_chunks(entries, MSM_MIN_CHUNK) + 1; };
+    auto chunks = [&](uint64_t entries) { return (uint64_t)msm_max_chunks(entries, chunk_floor); };
     b += 128 * (3 * Kw * 2 + chunks(ra * Ww) + chunks(rb * Ww) + chunks(rl * Ww)) + 256 * (Kw * 2 + chunks(rb * Ww));
     b += 128 * (Kh * 2 + chunks(n * Wh)) + (16ull << 20);
     return b;
@@ -553,7 +554,10 @@ int enqueue_witness_msms(g16_circuit* c, Workspace* ws, const void* d_w) {
     for (int i = 0; i < 4; i++) st[i] = c->serial ? ws->stream : ws->side[i];
     CK(cudaStreamWaitEvent(st[0], ws->ev_fork, 0), "stream wait");
     // one pass over the witness digits sorts the A, B and L live sets
-    for (auto& x : ws->sort_w) x.reduce_pieces = witness_reduce_pieces();
+    for (auto& x : ws->sort_w) {
+        x.reduce_pieces = witness_reduce_pieces();
+        x.chunk_floor = c->chunk_floor;
+    }
     MsmLiveSets sets;
     sets.count = 3;
     for (int j = 0; j < 3; j++) {
@@ -592,6 +596,7 @@ int enqueue_h_msm(g16_circuit* c, Workspace* ws, const void* d_h) {
     // the H reduction runs last on the main stream, mostly alone: shorter chains pay
     // (2^21 prove +0.5%, 2^18 +1.5%, 2^20 +1.3% against the 8192-piece default)
     ws->sort_h.reduce_pieces = MSM_REDUCE_PIECES_ALONE;
+    ws->sort_h.chunk_floor = c->chunk_floor;
     CK(msm_sort(ws->sort_h, d_h, c->h_count, true, c->c_h, st, c->tables, c->be->constant_work), "H sort");
     CK(msm_accumulate_g1(ws->sort_h, ws->acc[4], c->tables ? c->t_h : c->d_h, 0, nh, st), "H accumulate");
     const size_t bytes = ws->acc[4].result_bytes(XYZZ_G1_BYTES);
@@ -873,7 +878,8 @@ struct TuningLock {
                 w->graph = nullptr;
                 w->proofs = 0;
             }
-            c->ws_estimate = workspace_estimate(c->n_vars, c->n, c->c_w, c->c_h, c->rows[0], c->rows[1], c->rows[2], c->tables);
+            c->ws_estimate = workspace_estimate(c->n_vars, c->n, c->c_w, c->c_h, c->rows[0], c->rows[1], c->rows[2],
+                                                c->tables, c->chunk_floor);
         }
         {
             std::lock_guard<std::mutex> g(c->mu);
@@ -984,7 +990,9 @@ bool window_bits_ok(int b) { return b >= 8 && b <= 20; }
 // How a key is held (g16_plan_key): the window tables when the key, its tables
 // and one workspace fit in free_bytes, else the compact key (plain bases, one
 // bucket set per window) when it and one workspace fit, else DEVICE_MEMORY.
-// G16_CUDA_WINDOW_TABLES=0 takes the compact key whenever it fits.
+// G16_CUDA_WINDOW_TABLES=0 takes the compact key whenever it fits.  The
+// workspace counted is the smaller one, with chunks of MSM_CHUNK entries;
+// g16_prepare takes the larger where there is room for it.
 int plan_key(const g16_zkey_view& k, const uint32_t rows[3], uint64_t free_bytes, g16_key_plan* out) {
     const uint64_t nv = k.n_vars, n = k.domain_size;
     const uint64_t ra = rows[0], rb = rows[1], rl = rows[2];
@@ -1000,14 +1008,16 @@ int plan_key(const g16_zkey_view& k, const uint32_t rows[3], uint64_t free_bytes
     {
         const uint64_t Ww = (uint64_t)msm_windows(t.msm_window_bits_witness), Wh = (uint64_t)msm_windows(t.msm_window_bits_h);
         t.key_bytes = plain + (ra + rl) * Ww * 64 + rb * Ww * (64 + 128) + n * Wh * 64;
-        t.workspace_bytes = workspace_estimate(nv, n, t.msm_window_bits_witness, t.msm_window_bits_h, ra, rb, rl, true);
+        t.workspace_bytes = workspace_estimate(nv, n, t.msm_window_bits_witness, t.msm_window_bits_h, ra, rb, rl, true,
+                                               MSM_CHUNK);
     }
     g16_key_plan m = {};
     m.window_tables = 0;
     m.msm_window_bits_witness = msm_window_bits(std::max<uint64_t>(1, std::max(ra, std::max(rb, rl))));
     m.msm_window_bits_h = msm_window_bits(n);
     m.key_bytes = plain;
-    m.workspace_bytes = workspace_estimate(nv, n, m.msm_window_bits_witness, m.msm_window_bits_h, ra, rb, rl, false);
+    m.workspace_bytes = workspace_estimate(nv, n, m.msm_window_bits_witness, m.msm_window_bits_h, ra, rb, rl, false,
+                                           MSM_CHUNK);
     for (const g16_key_plan* p : {&t, &m}) {
         // sorted entries are 31-bit indices in either form
         const uint64_t Ww = (uint64_t)msm_windows(p->msm_window_bits_witness), Wh = (uint64_t)msm_windows(p->msm_window_bits_h);
@@ -1281,6 +1291,14 @@ int g16_prepare(g16_backend* b, const g16_zkey_view* k, g16_circuit** out) {
     c->rows_only = gnark;
     c->h_count = gnark ? n - 1 : n;
     for (int j = 0; j < 3; j++) c->rows[j] = live.rows[j];
+    // the spread accumulates' larger scratch only where a full pool of
+    // workspaces keeps its room: it never refuses a key or a proof in flight
+    const uint64_t spread = workspace_estimate(nv, n, c_w, c_h, live.rows[0], live.rows[1], live.rows[2], c->tables,
+                                               MSM_MIN_CHUNK);
+    if (plan.key_bytes + c->max_workspaces * spread <= free_bytes) {
+        c->chunk_floor = MSM_MIN_CHUNK;
+        c->ws_estimate = spread;
+    }
     if (const char* g = std::getenv("G16_CUDA_GRAPHS")) c->graphs = std::strcmp(g, "0") != 0;
     while ((1u << c->log_n) < n) c->log_n++;
     if (!unpack(c->alpha1, k->alpha_g1) || !unpack(c->beta1, k->beta_g1) || !unpack(c->delta1, k->delta_g1) ||

@@ -144,6 +144,7 @@ struct g16_circuit {
     std::vector<g16::Workspace*> idle;
     uint32_t max_workspaces = 8;
     uint64_t ws_estimate = 0;          // device bytes of one workspace, scratch included
+    uint32_t chunk_floor = g16::MSM_CHUNK;   // its MSMs' smallest accumulate chunk (MsmSort::chunk_floor)
     bool serial = false;               // every stage on one stream (profiling)
     bool graphs = true;                // replay proofs as captured CUDA graphs
     bool tuning = false;               // g16_autotune / g16_tuning_set running: no new proofs start

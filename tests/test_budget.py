@@ -1,0 +1,43 @@
+"""Device-memory budgets.  The short accumulate chunks that spread a small MSM over
+the SMs take more scratch (up to 58 MB a proof); a budget that holds a key with the
+ordinary chunks of 16 entries still does, and its proofs are the same."""
+import random
+
+import pytest
+
+import oracle as O
+import snarkrs_b200 as S
+
+
+def _key(constraints):
+    sc = S.SynthCircuit(seed=901, n_constraints=constraints, n_inputs=24, n_public=5)
+    return sc, sc.zkey(902)
+
+
+# the compact key with one workspace whose buffers hold one partial sum per 16 entries
+@pytest.mark.parametrize("constraints,held", [(500, 22826468), (2000, 28253804), (8000, 55056932),
+                                              (20000, 108306692)])
+def test_short_chunks_do_not_refuse_a_key(constraints, held):
+    pk = S.ProvingKey.from_bytes(_key(constraints)[1], check_points=False)
+    pk.plan(held)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tables", [True, False], ids=["tables", "compact"])
+def test_proofs_within_the_least_budget_equal_the_oracle(tables):
+    sc, zk = _key(3000)
+    pk, ok = S.ProvingKey.from_bytes(zk), O.Zkey(zk)
+    full = pk.plan(1 << 40)
+    limit = full["key_bytes"] + full["workspace_bytes"]
+    b = S.CudaBackend(0, vram_limit=limit if tables else limit - 1)
+    c = b.prepare(pk)
+    assert bool(c.window_tables()) == tables
+    held, rng = c.device_bytes(), random.Random(5)
+    for k in range(3):   # the third proof replays a captured graph
+        w = sc.witness(k)
+        r, s = (O.to_bytes(O.to_mont(rng.randrange(1, O.R_MOD))) for _ in range(2))
+        assert c.prove_with_blinders(w, r, s).to_bytes() == ok.prove(w, O.from_bytes(r), O.from_bytes(s))
+    assert c.device_bytes() - held == (full if tables else pk.plan(limit - 1))["workspace_bytes"]   # one workspace
+    c.close()
+    b.close()
+    ok.close()
