@@ -156,8 +156,9 @@ namespace {
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// Device bytes a plan for these jobs takes, for the budget check before any allocation.
-uint64_t plan_estimate(g16_circuit* const* cs, size_t count) {
+// Device bytes a plan for these jobs takes, for the budget check before any
+// allocation; chunk_floor: the spaces' smallest accumulate chunk.
+uint64_t plan_estimate(g16_circuit* const* cs, size_t count, uint32_t chunk_floor) {
     uint64_t b = 0;
     for (size_t j = 0; j < count; j++) {
         const g16_circuit* c = cs[j];
@@ -170,8 +171,9 @@ uint64_t plan_estimate(g16_circuit* const* cs, size_t count) {
         b += (Kw * 2 + c->rows[1] * Ww / 16) * XYZZ_G2_BYTES;
         b += (Kh * 2 + eh / 16) * XYZZ_G1_BYTES;
     }
-    // the spaces' smallest chunk counts (msm_max_chunks) past the sixteenths above
-    return b + (8ull << 20) + MSM_SPREAD_THREADS * (2 * XYZZ_G1_BYTES + XYZZ_G2_BYTES);
+    // short chunks: msm_max_chunks of the two G1 spaces and the G2 one, past the sixteenths above
+    if (chunk_floor < MSM_CHUNK) b += MSM_SPREAD_THREADS * (2 * XYZZ_G1_BYTES + XYZZ_G2_BYTES);
+    return b + (8ull << 20);
 }
 
 // device buffer that only grows, reallocated in stream order on st (the engine
@@ -444,9 +446,21 @@ struct BatchUsers {
 };
 
 // Layout E for the batch, its grow-only buffers counted against the backend's
-// device budget; on failure E keeps no layout.
+// device budget; on failure E keeps no layout.  The accumulates' chunks go below
+// MSM_CHUNK entries where the engine already holds the larger scratch, or where
+// it has to grow anyway and the budget has room for every engine's; so the
+// larger scratch refuses no batch that fits with chunks of MSM_CHUNK, and an
+// engine sized for a batch never grows for it.
 int layout_engine(g16_backend* b, BatchEngine& E, g16_circuit* const* cs, size_t count) {
-    const uint64_t need = plan_estimate(cs, count);
+    uint64_t need = plan_estimate(cs, count, MSM_CHUNK);
+    const uint64_t spread = plan_estimate(cs, count, MSM_MIN_CHUNK);
+    uint32_t floor = MSM_CHUNK;
+    if (spread <= E.accounted ||
+        (need > E.accounted && b->vram_used + batch_max_engines() * spread <= b->vram_limit)) {
+        floor = MSM_MIN_CHUNK;
+        need = spread;
+    }
+    for (MsmSpace* sp : {&E.g1, &E.g2, &E.hs}) sp->sort.chunk_floor = floor;
     if (need > E.accounted) {   // the engine's buffers grow: check and count the difference
         if (b->vram_used + (need - E.accounted) > b->vram_limit)
             return fail(G16_ERR_DEVICE_MEMORY, "batch of %zu proofs needs about %llu MiB of device memory", count,

@@ -41,3 +41,34 @@ def test_proofs_within_the_least_budget_equal_the_oracle(tables):
     c.close()
     b.close()
     ok.close()
+
+
+@pytest.mark.gpu
+def test_short_chunks_do_not_refuse_a_batch(backend):
+    """One engine's working set with chunks of 16 entries: what the reservation of an
+    unlimited backend counts, less the short chunks' 75776 partial sums in each space."""
+    sc, zk = _key(3000)
+    pk, n = S.ProvingKey.from_bytes(zk), 12
+    circ = backend.prepare(pk)
+    engines = 4
+    sized = S.CudaBackend(0)
+    c = sized.prepare(pk)
+    key = sized.vram_used()
+    sized.batch_reserve([c] * n)
+    need = (sized.vram_used() - key) // engines - 75776 * (2 * 128 + 256)
+    c.close()
+    sized.close()
+    b = S.CudaBackend(0, vram_limit=key + engines * need)
+    c = b.prepare(pk)
+    b.batch_reserve([c] * n)
+    rng = random.Random(6)
+    jobs = [(sc.witness(k),) + tuple(O.to_bytes(O.to_mont(rng.randrange(1, O.R_MOD))) for _ in range(2))
+            for k in range(n)]
+    want = [circ.prove_with_blinders(*j) for j in jobs]
+    allocs = S.device_alloc_count()
+    for _ in range(3):   # laid out, captured, replayed
+        assert b.prove_batch([(c,) + j for j in jobs]) == want
+    assert S.device_alloc_count() == allocs
+    c.close()
+    b.close()
+    circ.close()
