@@ -53,6 +53,15 @@ inline NttTiling ntt_default_tiling(uint32_t log_n) {
     return t;
 }
 
+// The tilings that g16_autotune times: every tile from the smallest default up
+// to the largest, with rows of 2, 4 and 8 columns.
+inline std::vector<NttTiling> ntt_tiling_candidates() {
+    std::vector<NttTiling> v;
+    for (uint32_t t = 8; t <= NTT_MAX_TILE_LOG; t++)
+        for (uint32_t l = 1; l <= 3; l++) v.push_back({t, l});
+    return v;
+}
+
 // The passes of a transform of 2^log_n under a tiling (host arithmetic only, so
 // that the kernels' indexing can be checked against it on the CPU): the inner
 // pass covers stages [0, k0) on contiguous tiles of 2^k0; each outer pass covers

@@ -2004,18 +2004,17 @@ int g16_autotune(g16_circuit* c, const uint8_t* w, size_t n, int concurrency, g1
     {
         NttTiling best = c->ntt.tiling;
         double best_t = -1;
-        for (uint32_t tl : {8u, 9u, 10u, 11u})
-            for (uint32_t ll : {2u, 3u}) {
-                if ((uint32_t)c->log_n <= 10 && !(tl == best.tile_log && ll == best.outer_log_l)) continue;
-                c->ntt.tiling = {tl, ll};
-                double t = together ? whole()
-                                    : time_on_stream(ws, reps, [&] { return run_h(c, ws, ws->d_w, ws->d_hpoly); });
-                if (t < 0) return G16_ERR_DEVICE;
-                if (best_t < 0 || t < best_t) {
-                    best_t = t;
-                    best = c->ntt.tiling;
-                }
+        for (const NttTiling& tl : ntt_tiling_candidates()) {
+            if ((uint32_t)c->log_n <= 10 && !(tl.tile_log == best.tile_log && tl.outer_log_l == best.outer_log_l)) continue;
+            c->ntt.tiling = tl;
+            double t = together ? whole()
+                                : time_on_stream(ws, reps, [&] { return run_h(c, ws, ws->d_w, ws->d_hpoly); });
+            if (t < 0) return G16_ERR_DEVICE;
+            if (best_t < 0 || t < best_t) {
+                best_t = t;
+                best = tl;
             }
+        }
         c->ntt.tiling = best;
     }
     // 2. H MSM window (H from the tiling just chosen is in d_hpoly)

@@ -327,3 +327,31 @@ def test_batched_h_pipelines_give_the_oracle_h(batch_plans):
                     assert i == j or w not in r, (batch, kind, jobs[i], jobs[j])
         for item in range(len(batch)):
             assert vecs[item][3] == want[item], (batch, item)
+
+
+CANDIDATES_PROBE = r"""
+#include <cstdio>
+#include "ntt.cuh"
+int main() {
+    for (auto& t : g16::ntt_tiling_candidates())
+        printf("%u %u %d\n", t.tile_log, t.outer_log_l, g16::ntt_tiling_valid(t) ? 1 : 0);
+    for (unsigned n = 1; n <= 27; n++) printf("%u %u -1\n", g16::ntt_default_tiling(n).tile_log, g16::ntt_default_tiling(n).outer_log_l);
+    return 0;
+}
+"""
+
+
+def test_autotuner_candidates_cover_the_tilings(tmp_path):
+    """The autotuner times every default tiling, and tiles of 2^10 to 2^12 with rows of 2, 4 and 8 columns."""
+    if shutil.which("nvcc") is None:
+        pytest.skip("nvcc not on PATH")
+    src, exe = tmp_path / "probe.cu", tmp_path / "probe"
+    src.write_text(CANDIDATES_PROBE)
+    subprocess.run(["nvcc", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "snarkrs_b200", "csrc"), "-I",
+                    os.path.join(ROOT, "include"), "-o", str(exe), str(src)], check=True, capture_output=True)
+    rows = [tuple(map(int, x.split())) for x in subprocess.run([str(exe)], capture_output=True, text=True,
+                                                                check=True).stdout.splitlines()]
+    candidates = {(t, l) for t, l, valid in rows if valid >= 0}
+    assert all(valid for _, _, valid in rows)
+    assert candidates >= {(t, l) for t, l, valid in rows if valid < 0}
+    assert candidates >= {(t, l) for t in (10, 11, 12) for l in (1, 2, 3)}
