@@ -76,6 +76,8 @@ constexpr uint64_t msm_reduce_pieces(bool shared_windows) {
 #endif
 constexpr uint32_t MSM_REDUCE_LB_G1 = G16_REDUCE_LB_G1;
 constexpr uint32_t MSM_REDUCE_LB_G2 = G16_REDUCE_LB_G2;
+static_assert(MSM_REDUCE_LB_G1 >= 2 && MSM_REDUCE_LB_G1 <= 7 && MSM_REDUCE_LB_G2 >= 1 && MSM_REDUCE_LB_G2 <= 6,
+              "a reduction block has 8 (G1) or 16 (G2) lanes a piece: 32 to 1024 threads");
 
 struct MsmReducePlan {
     uint32_t sets = 0, B = 0, seg = 1, lb = MSM_REDUCE_LB_G1, nb = 1, hb = 0;

@@ -340,3 +340,19 @@ def test_reduction_algebra_by_integer_emulation(defines):
         assert any(s[2] > 1 for s in shapes) and any(s[2] == 1 for s in shapes)
     finally:
         shutil.rmtree(d, ignore_errors=True)
+
+
+@pytest.mark.parametrize("define,ok", [("G16_REDUCE_LB_G1=7", True), ("G16_REDUCE_LB_G1=8", False),
+                                       ("G16_REDUCE_LB_G1=1", False), ("G16_REDUCE_LB_G2=6", True),
+                                       ("G16_REDUCE_LB_G2=7", False), ("G16_REDUCE_LB_G2=0", False)])
+def test_block_sizes_that_cannot_launch_do_not_compile(tmp_path, define, ok):
+    # two groups of 4 (G1) or 8 (G2) lanes a piece, a block of one warp to 1024 threads
+    if shutil.which("nvcc") is None:
+        pytest.skip("nvcc not on PATH")
+    src = tmp_path / "probe.cu"
+    src.write_text('#include "msm.cuh"\nint main() { return 0; }\n')
+    r = subprocess.run(["nvcc", "-std=c++17", "-O0", "-D" + define, "-I", os.path.join(ROOT, "snarkrs_b200", "csrc"),
+                        "-I", os.path.join(ROOT, "include"), "-c", "-o", str(tmp_path / "probe.o"), str(src)],
+                       capture_output=True, text=True)
+    assert (r.returncode == 0) == ok, r.stderr
+    assert ok or "32 to 1024 threads" in r.stderr
