@@ -13,6 +13,8 @@ namespace g16d {
 using g16::MSM_DEAD;
 using g16::MSM_MAX_SETS;
 using g16::MSM_CHUNK;
+using g16::MSM_PLAN_TILE;
+using g16::MsmPlanGrid;
 using g16::MSM_SPREAD_THREADS;
 using g16::MSM_MAX_TARGETS;
 
@@ -293,11 +295,11 @@ __device__ __forceinline__ uint32_t min_chunk(uint32_t M, uint32_t floor) {
 }
 
 // ---- from bucket counts to the accumulate's plan, for up to MSM_MAX_SETS sorts a launch ----
-// Three kernels, blockIdx.y picking the sort, 1024 buckets per block: block sums
-// of the counts; offsets (and the scatter's cursors), the chunk length L, each
-// bucket's partial-sum count and the fat list; the partial sums' bases.  A
-// block adds up the block sums before its own itself (at most a few thousand
-// words from L2) instead of waiting for a kernel that scans them: three
+// Three kernels, blockIdx.y picking the sort, a block's buckets in tiles of 1024
+// (msm_plan_grid): block sums of the counts; offsets (and the scatter's cursors),
+// the chunk length L, each bucket's partial-sum count and the fat list; the
+// partial sums' bases.  A block adds up the block sums before its own itself (at
+// most 4096 words from L2) instead of waiting for a kernel that scans them: three
 // launches where scanning twice, copying and counting took eight a sort (a
 // prove's four sorts 32 launches and 0.21 ms serialised, now 6 and 0.05 ms).
 struct SortPlanArgs {
@@ -310,12 +312,18 @@ struct SortPlanArgs {
     uint32_t* total;      // [0] M, [1] partial sums, [2] fat buckets, [3] L
     uint32_t Ks, K;       // sorted and real buckets (the constant-work sink is sorted, never reduced)
     uint32_t L_floor;
+    MsmPlanGrid grid;     // of Ks
+    // this block's tiles
+    __device__ __forceinline__ uint32_t first_tile() const { return blockIdx.x * grid.per_block; }
+    __device__ __forceinline__ uint32_t end_tile() const {
+        const uint32_t e = first_tile() + grid.per_block;
+        return e < grid.tiles ? e : grid.tiles;
+    }
 };
 struct SortPlanSets {
     SortPlanArgs s[MSM_MAX_SETS];
     uint32_t wave;
 };
-constexpr uint32_t PLAN_BLOCK = 1024;   // buckets per block of 256 threads
 
 // sums[0 .. b) and sums[0 .. nb), by the whole block
 __device__ __forceinline__ uint32_t sums_before(const uint32_t* sums, uint32_t b, uint32_t nb, uint32_t* warp_tot,
@@ -335,12 +343,14 @@ __device__ __forceinline__ uint32_t sums_before(const uint32_t* sums, uint32_t b
 
 __global__ void __launch_bounds__(256) k_plan_sums(SortPlanSets a) {
     const SortPlanArgs& s = a.s[blockIdx.y];
-    const size_t base = (size_t)blockIdx.x * PLAN_BLOCK + threadIdx.x * 4;
-    if (blockIdx.x && (size_t)blockIdx.x * PLAN_BLOCK >= s.Ks) return;   // uniform across the block
+    if (blockIdx.x >= s.grid.blocks) return;   // uniform across the block
     __shared__ uint32_t wt[32];
     uint32_t v = 0, total;
+    for (uint32_t tile = s.first_tile(); tile < s.end_tile(); tile++) {
+        const size_t base = (size_t)tile * MSM_PLAN_TILE + threadIdx.x * 4;
 #pragma unroll
-    for (int j = 0; j < 4; j++) v += base + j < s.Ks ? s.counts[base + j] : 0;
+        for (int j = 0; j < 4; j++) v += base + j < s.Ks ? s.counts[base + j] : 0;
+    }
     block_excl_scan(v, wt, total);
     if (threadIdx.x == 0) {
         s.sums[blockIdx.x] = total;
@@ -350,31 +360,34 @@ __global__ void __launch_bounds__(256) k_plan_sums(SortPlanSets a) {
 
 __global__ void __launch_bounds__(256) k_plan_offsets(SortPlanSets a) {
     const SortPlanArgs& s = a.s[blockIdx.y];
-    const size_t base = (size_t)blockIdx.x * PLAN_BLOCK + threadIdx.x * 4;
-    if (blockIdx.x && (size_t)blockIdx.x * PLAN_BLOCK >= s.Ks) return;   // uniform across the block
+    if (blockIdx.x >= s.grid.blocks) return;   // uniform across the block
     __shared__ uint32_t wt[32];
-    const uint32_t nb = (s.Ks + PLAN_BLOCK - 1) / PLAN_BLOCK;
-    uint32_t M, total, v[4], sum = 0;
-    const uint32_t before = sums_before(s.sums, blockIdx.x, nb, wt, M);
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        v[j] = base + j < s.Ks ? s.counts[base + j] : 0;
-        sum += v[j];
-    }
-    uint32_t off = before + block_excl_scan(sum, wt, total);
+    const uint32_t nb = s.grid.blocks;
+    uint32_t M, total, segs = 0;
+    uint32_t before = sums_before(s.sums, blockIdx.x, nb, wt, M);
     const uint32_t L = chunk_len(M, s.K, min_chunk(M, s.L_floor), a.wave);
-    uint32_t segs = 0;
+    for (uint32_t tile = s.first_tile(); tile < s.end_tile(); tile++) {
+        const size_t base = (size_t)tile * MSM_PLAN_TILE + threadIdx.x * 4;
+        uint32_t v[4], sum = 0;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const size_t g = base + j;
-        if (g >= s.Ks) break;
-        s.offsets[g] = off;
-        s.cursor[g] = off;
-        const uint32_t hi = off + v[j], ns = v[j] ? ((hi - 1) / L - off / L + 1) : 0;
-        s.counts[g] = ns;
-        if (g < s.K && ns > FAT_PARTIALS) s.fat_list[atomicAdd(s.total + 2, 1u)] = (uint32_t)g;
-        off = hi;
-        segs += ns;
+        for (int j = 0; j < 4; j++) {
+            v[j] = base + j < s.Ks ? s.counts[base + j] : 0;
+            sum += v[j];
+        }
+        uint32_t off = before + block_excl_scan(sum, wt, total);
+        before += total;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const size_t g = base + j;
+            if (g >= s.Ks) break;
+            s.offsets[g] = off;
+            s.cursor[g] = off;
+            const uint32_t hi = off + v[j], ns = v[j] ? ((hi - 1) / L - off / L + 1) : 0;
+            s.counts[g] = ns;
+            if (g < s.K && ns > FAT_PARTIALS) s.fat_list[atomicAdd(s.total + 2, 1u)] = (uint32_t)g;
+            off = hi;
+            segs += ns;
+        }
     }
     block_excl_scan(segs, wt, total);
     if (threadIdx.x == 0) {
@@ -389,23 +402,27 @@ __global__ void __launch_bounds__(256) k_plan_offsets(SortPlanSets a) {
 
 __global__ void __launch_bounds__(256) k_plan_segments(SortPlanSets a) {
     const SortPlanArgs& s = a.s[blockIdx.y];
-    const size_t base = (size_t)blockIdx.x * PLAN_BLOCK + threadIdx.x * 4;
-    if (blockIdx.x && (size_t)blockIdx.x * PLAN_BLOCK >= s.Ks) return;   // uniform across the block
+    if (blockIdx.x >= s.grid.blocks) return;   // uniform across the block
     __shared__ uint32_t wt[32];
-    const uint32_t nb = (s.Ks + PLAN_BLOCK - 1) / PLAN_BLOCK;
-    uint32_t S, total, v[4], sum = 0;
-    const uint32_t before = sums_before(s.sums + nb, blockIdx.x, nb, wt, S);
+    const uint32_t nb = s.grid.blocks;
+    uint32_t S, total;
+    uint32_t before = sums_before(s.sums + nb, blockIdx.x, nb, wt, S);
+    for (uint32_t tile = s.first_tile(); tile < s.end_tile(); tile++) {
+        const size_t base = (size_t)tile * MSM_PLAN_TILE + threadIdx.x * 4;
+        uint32_t v[4], sum = 0;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        v[j] = base + j < s.Ks ? s.counts[base + j] : 0;
-        sum += v[j];
-    }
-    uint32_t off = before + block_excl_scan(sum, wt, total);
+        for (int j = 0; j < 4; j++) {
+            v[j] = base + j < s.Ks ? s.counts[base + j] : 0;
+            sum += v[j];
+        }
+        uint32_t off = before + block_excl_scan(sum, wt, total);
+        before += total;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        if (base + j >= s.Ks) break;
-        s.seg_base[base + j] = off;
-        off += v[j];
+        for (int j = 0; j < 4; j++) {
+            if (base + j >= s.Ks) break;
+            s.seg_base[base + j] = off;
+            off += v[j];
+        }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         s.total[1] = S;
@@ -1272,7 +1289,7 @@ static cudaError_t grow_bytes(cudaStream_t st, void*& p, size_t& cap, size_t nee
 }
 
 // Scratch words for a plan over Ks buckets: two block sums each.
-static size_t plan_tmp_words(size_t Ks) { return 2 * ((Ks + PLAN_BLOCK - 1) / PLAN_BLOCK); }
+static size_t plan_tmp_words(size_t Ks) { return 2 * (size_t)msm_plan_grid(Ks).blocks; }
 
 // The accumulate's plan from the bucket counts of `count` sorts (d_counts
 // filled); the scatter follows.
@@ -1283,8 +1300,8 @@ static cudaError_t sort_plan(MsmSort* const* sorts, int count, cudaStream_t st) 
     for (int j = 0; j < count; j++) {
         const MsmSort& s = *sorts[j];
         a.s[j] = {s.d_counts, s.d_offsets, s.d_cursor, s.d_seg_base, s.d_fat_list, s.d_scan_tmp, s.d_total, s.Ks, s.K,
-                  s.chunk};
-        nb = std::max(nb, (s.Ks + PLAN_BLOCK - 1) / PLAN_BLOCK);
+                  s.chunk, msm_plan_grid(s.Ks)};
+        nb = std::max(nb, a.s[j].grid.blocks);
     }
     const dim3 grid(nb, count);
     {

@@ -162,6 +162,25 @@ constexpr size_t msm_max_chunks(size_t max_entries, uint32_t floor) {
     return whole > spread ? whole : spread;
 }
 
+// Blocks of the kernels that turn bucket counts into the accumulate's plan
+// (k_plan_* in msm.cu): a tile of 1024 buckets each, several once the tiles pass
+// 4096 (from 2^22 buckets on), since every block adds up all blocks' sums and the
+// step would otherwise grow with the square of the buckets.
+constexpr uint32_t MSM_PLAN_TILE = 1024;
+constexpr uint32_t MSM_PLAN_BLOCKS = 4096;
+struct MsmPlanGrid {
+    uint32_t tiles, per_block, blocks;
+};
+constexpr MsmPlanGrid msm_plan_grid(size_t buckets) {
+    MsmPlanGrid g = {};
+    g.tiles = (uint32_t)((buckets + MSM_PLAN_TILE - 1) / MSM_PLAN_TILE);
+    g.per_block = (g.tiles + MSM_PLAN_BLOCKS - 1) / MSM_PLAN_BLOCKS;
+    if (!g.per_block) g.per_block = 1;
+    g.blocks = (g.tiles + g.per_block - 1) / g.per_block;
+    if (!g.blocks) g.blocks = 1;   // no bucket: the totals are still written
+    return g;
+}
+
 struct MsmSort {
     // parameters
     int c = 0, W = 0;

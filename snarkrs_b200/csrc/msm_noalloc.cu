@@ -63,7 +63,7 @@ constexpr size_t OFF_CURSOR = OFF_OFFSETS + U32_K;
 constexpr size_t OFF_SEGBASE = OFF_CURSOR + U32_K;
 constexpr size_t OFF_FAT = OFF_SEGBASE + U32_K;
 constexpr size_t OFF_SCANTMP = OFF_FAT + U32_K;
-constexpr size_t SCANTMP_ELEMS = 2 * ((NOALLOC_K + 1023) / 1024);
+constexpr size_t SCANTMP_ELEMS = 2 * g16::msm_plan_grid(NOALLOC_K).blocks;
 constexpr size_t OFF_ENTRIES = align256(OFF_SCANTMP + 4 * SCANTMP_ELEMS);
 constexpr size_t ENTRIES_ELEMS = NOALLOC_MAX_POINTS * NOALLOC_W;
 constexpr size_t OFF_TOTAL = align256(OFF_ENTRIES + 4 * ENTRIES_ELEMS);

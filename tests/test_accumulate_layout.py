@@ -7,8 +7,14 @@ its own slot of its bucket's range, every slot is written once, the fat-bucket
 jobs and the bucket sums give each bucket the sum of its entries, and the chunk
 length keeps the thread count within its cap.  The GPU parity tests check the
 CUDA code itself."""
+import os
 import random
+import shutil
+import subprocess
 
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 ACC_THREADS = 1 << 19
 FAT_PARTIALS, FAT_JOBS, FAT_JOB_MIN = 16, 64, 128
 
@@ -127,3 +133,36 @@ def test_chunk_len_cases():
     assert chunk_len(M, 1 << 20, 16, wave) == 20
     M = int(2.97 * wave * 16)                                 # 3 waves of 16 against 2 of 24: kept
     assert chunk_len(M, 1 << 20, 16, wave) == 16
+
+
+GRID_PROBE = r"""
+#include <cstdio>
+#include "msm.cuh"
+int main() {
+    unsigned long long k;
+    while (scanf("%llu", &k) == 1) {
+        const g16::MsmPlanGrid g = g16::msm_plan_grid(k);
+        printf("%u %u %u\n", g.tiles, g.per_block, g.blocks);
+    }
+    return 0;
+}
+"""
+
+
+def test_plan_blocks_read_a_bounded_number_of_sums(tmp_path):
+    """Every block of the plan kernels adds up all blocks' sums: their number stays at
+    4096 however many buckets there are, and the blocks' tiles cover each bucket once."""
+    if shutil.which("nvcc") is None:
+        pytest.skip("nvcc not on PATH")
+    src, exe = tmp_path / "probe.cu", tmp_path / "probe"
+    src.write_text(GRID_PROBE)
+    subprocess.run(["nvcc", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "snarkrs_b200", "csrc"), "-I",
+                    os.path.join(ROOT, "include"), "-o", str(exe), str(src)], check=True, capture_output=True)
+    ks = [0, 1, 1023, 1024, 1025, 24576, 1 << 22, (1 << 22) + 1, 13 << 19, (13 << 19) + 1, 1 << 25, (1 << 31) - 1]
+    out = subprocess.run([str(exe)], input=" ".join(map(str, ks)), capture_output=True, text=True, check=True).stdout
+    for k, line in zip(ks, out.splitlines()):
+        tiles, per, blocks = map(int, line.split())
+        assert tiles == (k + 1023) // 1024 and 1 <= blocks <= 4096
+        assert (per == 1) == (tiles <= 4096)
+        covered = [t for b in range(blocks) for t in range(b * per, min((b + 1) * per, tiles))]
+        assert covered == list(range(tiles))

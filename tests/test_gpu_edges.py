@@ -78,3 +78,25 @@ def test_ntt_tilings(S, O, backend, log_n):
     assert ntt.ntt(data) == O.ntt(log_n, O.NTT_FORWARD, data)
     assert ntt.intt_coset_ntt(data) == O.ntt(log_n, O.NTT_INTT_COSET_NTT, data)
     assert ntt.coset_ntt(data, inverse=True) == O.ntt(log_n, O.NTT_COSET_INVERSE, data)
+
+
+@pytest.mark.parametrize("constant_work", [False, True])
+def test_millions_of_buckets(S, O, constant_work):
+    """A compact key at 20-bit windows sorts into 13 x 2^19 buckets (one more with constant
+    work), past the 2^22 where a block of the plan kernels takes several tiles of them."""
+    sc = S.SynthCircuit(seed=31, n_constraints=700, n_inputs=24, n_public=5)
+    zk = sc.zkey(32)
+    ok = O.Zkey(zk)
+    os.environ["G16_CUDA_WINDOW_TABLES"] = "0"
+    try:
+        b = S.CudaBackend(0, constant_work=constant_work)
+        c = b.prepare(S.ProvingKey.from_bytes(zk))
+    finally:
+        del os.environ["G16_CUDA_WINDOW_TABLES"]
+    t = c.tuning()
+    c.set_tuning(20, 20, t["ntt_tile_log"], t["ntt_outer_log_l"])
+    w, (r, s) = sc.witness(3), [O.to_bytes(O.to_mont(x)) for x in (1234567, 7654321)]
+    assert c.prove_with_blinders(w, r, s).to_bytes() == ok.prove(w, O.from_bytes(r), O.from_bytes(s))
+    c.close()
+    b.close()
+    ok.close()
