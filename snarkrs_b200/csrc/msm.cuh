@@ -295,9 +295,8 @@ constexpr size_t XYZZ_G2_BYTES = 256;
 
 // The prover reads each of its five MSM results (a sum per bucket set) back into
 // a pinned host slot of this many bytes: one bucket set with window tables, one
-// per window with a compact key.
+// per window with a compact key, at most 32 of them (8-bit windows).
 constexpr size_t MSM_RESULT_SLOT_BYTES = 32 * 256;
-constexpr size_t MSM_RESULT_SLOT_COMPACT_BYTES = 128 * 1024;
 
 // ---- batched MSMs (many MSMs in one launch per step) ----
 // A space holds the buckets of many MSMs of one group (segments) back to back;

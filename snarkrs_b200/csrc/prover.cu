@@ -355,9 +355,6 @@ int build_h_table(g16_circuit* c, int ch, cudaStream_t st) {
     return G16_OK;
 }
 
-// Host readback slot of one MSM's reduction terms (sizes checked against every
-// window width by tests/test_reduce_plan.py).
-constexpr size_t WIN_SLOT_COMPACT = MSM_RESULT_SLOT_COMPACT_BYTES;
 // Bucket-reduction piece target of the witness MSMs (0: the library default for
 // MSMs whose reductions run beside other work); G16_WITNESS_REDUCE_PIECES overrides it.
 uint64_t witness_reduce_pieces() {
@@ -367,8 +364,6 @@ uint64_t witness_reduce_pieces() {
     }();
     return v;
 }
-
-size_t win_slot(const g16_circuit* c) { return c->tables ? MSM_RESULT_SLOT_BYTES : WIN_SLOT_COMPACT; }
 
 // Take an idle workspace, or build one while the pool is below its cap and the
 // backend's device-memory budget has room; otherwise wait for one to come back.
@@ -387,7 +382,7 @@ int acquire(g16_circuit* c, Workspace** out) {
         bool room = c->be->vram_used + c->ws_estimate <= c->be->vram_limit;
         if (c->pool.size() < c->max_workspaces && (room || c->pool.empty())) {
             auto ws = std::make_unique<Workspace>();
-            cudaError_t e = ws->init(c->n_vars, c->n, win_slot(c));
+            cudaError_t e = ws->init(c->n_vars, c->n);
             if (e == cudaSuccess) {
                 c->device_bytes += c->ws_estimate;
                 c->be->vram_used += c->ws_estimate;
@@ -546,7 +541,7 @@ int fork_witness(Workspace* ws) {
     return G16_OK;
 }
 int enqueue_witness_msms(g16_circuit* c, Workspace* ws, const void* d_w) {
-    const size_t WIN_SLOT = ws->win_slot;
+    constexpr size_t WIN_SLOT = MSM_RESULT_SLOT_BYTES;
     // window tables: entry w rows + rank of a table of rows W points; compact:
     // entry rank of the plain bases
     const uint32_t W = c->tables ? (uint32_t)msm_windows(c->c_w) : 1u;
@@ -590,7 +585,7 @@ int enqueue_witness_msms(g16_circuit* c, Workspace* ws, const void* d_w) {
 }
 
 int enqueue_h_msm(g16_circuit* c, Workspace* ws, const void* d_h) {
-    const size_t WIN_SLOT = ws->win_slot;
+    constexpr size_t WIN_SLOT = MSM_RESULT_SLOT_BYTES;
     cudaStream_t st = ws->stream;
     const uint32_t nh = c->h_count * (c->tables ? (uint32_t)msm_windows(c->c_h) : 1u);
     // the H reduction runs last on the main stream, mostly alone: shorter chains pay
@@ -615,7 +610,7 @@ int enqueue_join(Workspace* ws) {
 }
 
 int collect_msms(g16_circuit* c, Workspace* ws, MsmJac& out) {
-    const size_t WIN_SLOT = ws->win_slot;
+    constexpr size_t WIN_SLOT = MSM_RESULT_SLOT_BYTES;
     CK(cudaStreamSynchronize(ws->stream), "MSM stages");
     timer().collect();
     {
@@ -858,7 +853,7 @@ struct TuningLock {
             }
             if (c->pool.size() >= c->max_workspaces || c->be->vram_used + c->ws_estimate > c->be->vram_limit) break;
             auto w = std::make_unique<Workspace>();
-            if (w->init(c->n_vars, c->n, win_slot(c)) != cudaSuccess) {
+            if (w->init(c->n_vars, c->n) != cudaSuccess) {
                 w->release();
                 cudaGetLastError();
                 break;
@@ -1550,7 +1545,7 @@ int g16_circuit_warm(g16_circuit* c, uint32_t count) {
                 c->idle.pop_back();
             } else if (c->pool.size() < c->max_workspaces && c->be->vram_used + c->ws_estimate <= c->be->vram_limit) {
                 auto w = std::make_unique<Workspace>();
-                cudaError_t e = w->init(c->n_vars, c->n, win_slot(c));
+                cudaError_t e = w->init(c->n_vars, c->n);
                 if (e != cudaSuccess) {
                     w->release();
                     cudaGetLastError();

@@ -64,14 +64,12 @@ struct Workspace {
     bool graph_constant_work = false;  // the mode the graph was captured in
     uint64_t proofs = 0;
     uint64_t bytes = 0;                // fixed device buffers
-    size_t win_slot = 0;               // bytes of h_win per MSM
 
-    cudaError_t init(uint32_t n_vars, uint32_t n, size_t slot) {
-        win_slot = slot;
+    cudaError_t init(uint32_t n_vars, uint32_t n) {
         cudaError_t e = g16::dev_malloc(&d_w, 32ull * n_vars);
         if (e == cudaSuccess) e = g16::dev_malloc(&d_abc, 32ull * n * 3);
         if (e == cudaSuccess) e = g16::dev_malloc(&d_hpoly, 32ull * n);
-        if (e == cudaSuccess) e = cudaMallocHost((void**)&h_win, 5 * slot);
+        if (e == cudaSuccess) e = cudaMallocHost((void**)&h_win, 5 * MSM_RESULT_SLOT_BYTES);
         if (e == cudaSuccess) e = cudaMallocHost((void**)&h_work, 16 * sizeof(unsigned long long));
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
         for (auto& x : side)
