@@ -4,8 +4,9 @@ snarkrs_b200/csrc/msm.cuh), compiled here by nvcc for the CPU.
 For every window width the prover and the standalone MSM can use, over G1 and
 G2 and both piece targets, the plan must cover every bucket exactly once
 (pieces x seg = B, blocks x 2^lb >= pieces), keep seg a power of two no larger
-than 32, take the direct path only for at most two blocks in all, and give a
-prover MSM result that fits the prover's readback slot per MSM (MSM_RESULT_SLOT_BYTES).
+than 32, take the direct path only for at most two blocks in all, and give the
+finish kernel no more bit terms than it has groups; a prover MSM's set sums fit
+its readback slot (MSM_RESULT_SLOT_BYTES).
 """
 import os
 import shutil
@@ -86,6 +87,14 @@ def test_results_fit_the_readback_slot(plan):
     plan([(1, 1, 0, 8192)])
     for c in range(8, 21):
         assert (255 + c - 1) // c * 256 <= plan.slot_bytes
+
+
+def test_finish_kernel_has_a_group_for_every_bit_term(plan):
+    # 32 groups: the bit terms, T in the last (window widths up to 24, any piece target)
+    cases = [(sets, 1 << (c - 1), g2, t) for c in range(4, 25) for sets in (1, (255 + c - 1) // c)
+             for g2 in (0, 1) for t in (1, 8192, 32768, 1 << 40)]
+    for _, p in zip(cases, plan(cases)):
+        assert p["lb"] + p["hb"] < 31
 
 
 LAYOUT_PROBE = r"""
@@ -208,98 +217,114 @@ def _plan_probe(defines):
     return run, d
 
 
+def _piece_block(S, g0s, seg, LB):
+    """reduce_piece_block: the block's LB + 2 points from its 2^LB pieces (g0s: a piece's
+    first bucket, None past the set's end).  Two groups a piece; slots are written only
+    by their own group, and no step may read a slot that another group writes in it."""
+    N, weighted = 1 << LB, seg > 1
+    first, second = [0] * N, [0] * N
+    nxt = [0 if g is None else S[g + seg - 1] for g in g0s]
+    for j in range(seg + 1 if weighted else 1):
+        second = [y + x for x, y in zip(first, second)]      # tot, one step behind run
+        first = [x + v for x, v in zip(first, nxt)]
+        nxt = [S[g + seg - 2 - j] if g is not None and j + 1 < seg else 0 for g in g0s]
+    acc = [list(first), list(second)]
+    slots = [list(first), list(second)]
+    lg = [t.bit_length() - 1 if t else 0 for t in range(N)]
+    for k in range(1, LB + 1):
+        h = N >> k
+        for half in (0, 1):
+            src = {}
+            for t in range(N):
+                if t < h:
+                    if not half or weighted:
+                        src[t] = t + h
+                elif t >= 2 * h and not half:
+                    hs, s = 1 << lg[t], 1 << (k - (LB - lg[t]) - 1)
+                    o = t - hs
+                    if o & (2 * s - 1) == 0 and o + s < hs:
+                        src[t] = t + s
+            assert not set(src) & set(src.values()), "a slot read in the step that writes it"
+            for t, x in src.items():
+                acc[half][t] += slots[half][x]
+            for t in src:
+                slots[half][t] = acc[half][t]
+    out = [None] * (LB + 2)
+    out[0] = acc[1][0] if weighted else acc[0][0]            # T
+    out[LB + 1] = acc[0][0]                                  # R
+    for t in range(1, N):
+        if t & (t - 1) == 0:
+            out[1 + lg[t]] = acc[0][t]                       # G_lg
+    return out
+
+
+def _set_term(points, base, nb, o, LB):
+    """reduce_set_term: one term of a set over its nb blocks."""
+    bits = o > LB
+    i, count = (o - LB - 1, nb // 2) if bits else (0, nb)
+    at = lambda x: ((x >> i) << (i + 1)) | (1 << i) | (x & ((1 << i) - 1)) if bits else x
+    js = [at(x) for x in range(count)]
+    assert js == [j for j in range(nb) if not bits or (j >> i) & 1]
+    return sum(points[base + j * (LB + 2) + (LB + 1 if bits else o)] for j in js)
+
+
+def _finish(points, base, LB, nb, hb, direct, seg):
+    """reduce_finish: 32 groups of lanes, the bit terms combined in a tree, T in the last."""
+    m, G = LB + hb, 32
+    assert m < G - 1 and (not direct or nb <= 2)
+    acc = [0] * G
+    for g in range(G):
+        is_t = g == G - 1
+        if not direct:
+            if g < m or is_t:
+                acc[g] = points[base + (0 if is_t else 1 + g)]
+            continue
+        low, o = is_t or g < LB, 0 if is_t else 1 + g
+        if low:
+            acc[g] = points[base + o]
+        elif g < m:
+            acc[g] = points[base + (LB + 2) + LB + 1]
+        if nb > 1 and low:
+            acc[g] += points[base + (LB + 2) + o]
+    smem, s = [None] * G, 1
+    while s < m:
+        for g in range(G):
+            if g & (2 * s - 1) == s and g < m:
+                acc[g] <<= s                                 # s doublings
+                assert smem[g] is None, "a slot written twice"
+                smem[g] = acc[g]
+        for g in range(G):
+            if g & (2 * s - 1) == 0 and g + s < m:
+                acc[g] += smem[g + s]
+        s *= 2
+    return acc[0] * seg + acc[G - 1]
+
+
 def _emulate_reduction(S, sets, B, p):
-    """k_reduce_pieces, k_reduce_sets and the host's set_sum (msm.cu) on integers standing
-    in for points (addition is +, doubling is *2), step by step as the kernels index them.
-    Returns each set's sum_b (b + 1) S_b as the device and host would form it."""
+    """k_reduce_pieces, k_reduce_sets and k_reduce_finish (msm.cu) on integers standing in
+    for points (an addition is +, a doubling *2), step by step as the kernels index them."""
     LB, seg, nb, hb = p["lb"], p["seg"], p["nb"], p["hb"]
-    N = 1 << LB
-    weighted = seg > 1
-    terms = LB + 2
-    blocks_out = [0] * (sets * nb * terms)
+    points = []
     for st in range(sets):
         for jb in range(nb):
-            run, tot = [0] * N, [0] * N
-            for t in range(N):
-                pc = jb * N + t
-                if pc * seg < B:
-                    g0 = st * B + pc * seg
-                    for i in range(seg - 1, -1, -1):
-                        run[t] += S[g0 + i]
-                        if weighted:
-                            tot[t] += run[t]
-            s_run, s_tot = list(run), list(tot)
-            lg = [0 if t == 0 else t.bit_length() - 1 for t in range(N)]
-            for k in range(1, LB + 1):
-                h = N >> k
-                r_run, r_tot = list(s_run), list(s_tot)   # a step reads the state the barrier left
-                for t in range(N):
-                    if t < h:
-                        run[t] = run[t] + r_run[t + h]
-                        s_run[t] = run[t]
-                    elif t < 2 * h:
-                        if weighted:
-                            tot[t] = r_tot[t - h] + r_tot[t]
-                            s_tot[t - h] = tot[t]
-                    else:
-                        hs, s = 1 << lg[t], 1 << (k - (LB - lg[t]) - 1)
-                        o = t - hs
-                        if (o & (2 * s - 1)) == 0 and o + s < hs:
-                            run[t] = run[t] + r_run[t + s]
-                            s_run[t] = run[t]
-            o0 = (st * nb + jb) * terms
-            for t in range(N):
-                if t == 0:
-                    if not weighted:
-                        blocks_out[o0] = run[0]
-                    blocks_out[o0 + LB + 1] = run[0]
-                elif t & (t - 1) == 0:
-                    blocks_out[o0 + 1 + lg[t]] = run[t]
-                    if t == 1 and weighted:
-                        blocks_out[o0] = tot[1]
-    sums = []
-    for st in range(sets):
-        base = st * nb * terms
-        if p["direct"]:
-            T, G, Gb = 0, [0] * LB, [0] * hb
-            for j in range(nb):
-                o = base + j * terms
-                T += blocks_out[o]
-                for i in range(LB):
-                    G[i] += blocks_out[o + 1 + i]
-                for i in range(hb):
-                    if (j >> i) & 1:
-                        Gb[i] += blocks_out[o + LB + 1]
-        else:   # k_reduce_sets: term o of the set over its nb blocks
-            res = []
-            for o in range(LB + 1 + hb):
-                acc = 0
-                for j in range(nb):
-                    if o <= LB:
-                        acc += blocks_out[base + j * terms + o]
-                    elif (j >> (o - LB - 1)) & 1:
-                        acc += blocks_out[base + j * terms + LB + 1]
-                res.append(acc)
-            T, G, Gb = res[0], res[1:1 + LB], res[LB + 1:]
-        acc = 0
-        for i in range(hb - 1, -1, -1):
-            acc = 2 * acc + Gb[i]
-        for j in range(LB - 1, -1, -1):
-            acc = 2 * acc + G[j]
-        s = seg
-        while s > 1:
-            acc *= 2
-            s >>= 1
-        sums.append(acc + T)
-    return sums
+            pieces = [(jb << LB) + t for t in range(1 << LB)]
+            points += _piece_block(S, [st * B + x * seg if x * seg < B else None for x in pieces], seg, LB)
+    assert None not in points and len(points) == p["block_points"]
+    stride = nb * (LB + 2)
+    if not p["direct"]:
+        points = [_set_term(points, st * stride, nb, o, LB) for st in range(sets) for o in range(LB + 1 + hb)]
+        stride = LB + 1 + hb
+    assert stride == p["set_terms"]
+    return [_finish(points, st * stride, LB, nb, hb, p["direct"], seg) for st in range(sets)]
 
 
 @pytest.mark.parametrize("defines", [[], ["-DG16_REDUCE_LB_G1=7", "-DG16_REDUCE_LB_G2=6"]],
-                         ids=["blocks-of-2^8", "blocks-of-2^7-and-2^6"])
+                         ids=["blocks-of-2^5-and-2^4", "blocks-of-2^7-and-2^6"])
 def test_reduction_algebra_by_integer_emulation(defines):
     # the pieces kernel's running sums, halvings and per-bit trees, the sets kernel and the
-    # host's combination give sum_b (b + 1) S_b for every plan shape: direct and summed on
-    # the device, weighted (seg > 1) and not, one or several sets
+    # finish kernel's tree give sum_b (b + 1) S_b for every plan shape: direct (one block a
+    # set, two blocks of one) and through the sets kernel, weighted (seg > 1) and not, one or
+    # several sets; and as a batched space runs it, which never takes the direct path
     if shutil.which("nvcc") is None:
         pytest.skip("nvcc not on PATH")
     import random
@@ -321,8 +346,11 @@ def test_reduction_algebra_by_integer_emulation(defines):
             S = [rng.randrange(1, 1 << 20) for _ in range(sets * B)]
             want = [sum((b + 1) * S[st * B + b] for b in range(B)) for st in range(sets)]
             assert _emulate_reduction(S, sets, B, p) == want, (sets, B, g2, target, p)
+            assert _emulate_reduction(S, sets, B, dict(p, direct=0, set_terms=p["lb"] + 1 + p["hb"])) == want
         assert any(s[4] == 1 for s in shapes) and any(s[4] == 0 for s in shapes)
         assert any(s[2] > 1 for s in shapes) and any(s[2] == 1 for s in shapes)
+        assert {s[3] for s in shapes if s[4]} == {1, 2}
+        assert any((s[5] + s[3].bit_length() - 1) & (s[5] + s[3].bit_length() - 2) for s in shapes)   # uneven trees
     finally:
         shutil.rmtree(d, ignore_errors=True)
 
