@@ -3,8 +3,8 @@
 The pass plan comes from the product's own host code (ntt_inner_k and
 ntt_outer_passes in ntt.cuh, compiled here by nvcc for the CPU).  The kernels'
 index arithmetic, restated here line for line from ntt.cu (the GPU parity tests
-check the CUDA code itself), is then replayed on integers mod r: run_stage's butterfly
-pairs and twiddle positions, ntt_pass_tile's tile-to-global mapping, the fused
+check the CUDA code itself), is then replayed on integers mod r: the butterflies and
+twiddle positions of run_stage and run_two_stages on a tile's permuted slots, ntt_pass_tile's tile-to-global mapping, the fused
 middle's DIF stages, coset multiply and DIT stages, and the launch order of
 ntt_intt_coset_ntt and ntt_h_pipeline (including the H = A*B - C join on the
 last pass).  Every valid tiling at small sizes must give the oracle's
@@ -68,25 +68,96 @@ def plans():
     shutil.rmtree(d, ignore_errors=True)
 
 
-def run_stage(dif, sm, j, s_lo, log_L, lo0, log_n, half_tile, tw):
-    L = 1 << log_L
-    s = s_lo + j
-    jmask = (1 << j) - 1
-    for q in range(half_tile):   # one butterfly per q; the pairs of a stage are disjoint
-        l, mq = q & (L - 1), q >> log_L
-        mid_a = ((mq >> j) << (j + 1)) | (mq & jmask)
-        ea = (mid_a << log_L) | l
+def slot(e):
+    return e ^ (((e >> 3) & 1) << 1) ^ (((e >> 4) & 1) * 5)
+
+
+class Tile:
+    """A shared-memory tile: the elements at their permuted slots."""
+
+    def __init__(self, values):
+        self.mem = [None] * len(values)
+        for e, x in enumerate(values):
+            self[e] = x
+
+    def __getitem__(self, e):
+        return self.mem[slot(e)]
+
+    def __setitem__(self, e, x):
+        self.mem[slot(e)] = x % R
+
+
+def butterfly(dif, a, b, tw, i):
+    if dif:
+        return a + b, (a - b) * (tw[i] if i else 1)
+    t = b * (tw[i] if i else 1)
+    return a + t, a - t
+
+
+def stage_elements(q, j, log_L, two):
+    """First element, lane column and mid of thread index q in run_stage / run_two_stages."""
+    l, mq = q & ((1 << log_L) - 1), q >> log_L
+    mid = ((mq >> j) << (j + (2 if two else 1))) | (mq & ((1 << j) - 1))
+    return (mid << log_L) | l, l, mid
+
+
+def run_stage(dif, t, j, s_lo, log_L, lo0, log_n, tile, tw):
+    s, jmask = s_lo + j, (1 << j) - 1
+    for q in range(tile // 2):   # one butterfly per q; the pairs of a stage are disjoint
+        ea, l, mid = stage_elements(q, j, log_L, False)
         eb = ea + (1 << (j + log_L))
-        pos = ((mid_a & jmask) << s_lo) | (lo0 + l)
-        a, b = sm[ea], sm[eb]
-        w = tw[pos << (log_n - s - 1)]
+        pos = ((mid & jmask) << s_lo) | (lo0 + l)
+        t[ea], t[eb] = butterfly(dif, t[ea], t[eb], tw, pos << (log_n - s - 1))
+
+
+def run_two_stages(dif, t, j, s_lo, log_L, lo0, log_n, tile, tw):
+    s, jmask, step = s_lo + j, (1 << j) - 1, 1 << (j + log_L)
+    seen = set()
+    for q in range(tile // 4):   # four elements per q, disjoint
+        e, l, mid = stage_elements(q, j, log_L, True)
+        pos = ((mid & jmask) << s_lo) | (lo0 + l)
+        w0, w1 = pos << (log_n - s - 1), pos << (log_n - s - 2)
+        w2 = (pos + (1 << s)) << (log_n - s - 2)
+        at = [e, e + step, e + 2 * step, e + 3 * step]
+        assert not seen & set(at)
+        seen.update(at)
+        a, b, c, d = (t[x] for x in at)
         if dif:
-            d = a - b
-            a, b = a + b, (d * w if pos else d)
+            a, c = butterfly(True, a, c, tw, w1)
+            b, d = butterfly(True, b, d, tw, w2)
+            a, b = butterfly(True, a, b, tw, w0)
+            c, d = butterfly(True, c, d, tw, w0)
         else:
-            t = b * w if pos else b
-            a, b = a + t, a - t
-        sm[ea], sm[eb] = a % R, b % R
+            a, b = butterfly(False, a, b, tw, w0)
+            c, d = butterfly(False, c, d, tw, w0)
+            a, c = butterfly(False, a, c, tw, w1)
+            b, d = butterfly(False, b, d, tw, w2)
+        t[at[0]], t[at[1]], t[at[2]], t[at[3]] = a, b, c, d
+
+
+def run_stages(dif, t, k, s_lo, log_L, lo0, log_n, tw):
+    """Two stages at a time, or single ones where a block has a thread per butterfly: the
+    stage functions below a size depend on the launch, so the replay takes both in turn."""
+    tile = (1 << k) << log_L
+    pairs = k // 2 if run_stages.paired else 0
+    if dif:
+        for j in range(k - 1, 2 * pairs - 1, -1):
+            run_stage(True, t, j, s_lo, log_L, lo0, log_n, tile, tw)
+    for i in range(pairs):
+        run_two_stages(dif, t, 2 * (pairs - 1 - i) if dif else 2 * i, s_lo, log_L, lo0, log_n, tile, tw)
+    if not dif:
+        for j in range(2 * pairs, k):
+            run_stage(False, t, j, s_lo, log_L, lo0, log_n, tile, tw)
+
+
+run_stages.paired = True
+
+
+@pytest.fixture(params=[True, False], ids=["two-stages", "single-stages"])
+def stages(request):
+    run_stages.paired = request.param
+    yield request.param
+    run_stages.paired = True
 
 
 def pass_tile(dif, data, bx, log_n, s_lo, k, log_L, tw, join=None):
@@ -96,9 +167,8 @@ def pass_tile(dif, data, bx, log_n, s_lo, k, log_L, tw, join=None):
     assert bph >= 0
     hi, lo0 = bx >> bph, (bx & ((1 << bph) - 1)) << log_L
     gi = [(hi << (s_lo + k)) | ((e >> log_L) << s_lo) | (lo0 + (e & (L - 1))) for e in range(tile)]
-    sm = [data[g] for g in gi]
-    for jj in range(k):
-        run_stage(dif, sm, k - 1 - jj if dif else jj, s_lo, log_L, lo0, log_n, tile // 2, tw)
+    sm = Tile([data[g] for g in gi])
+    run_stages(dif, sm, k, s_lo, log_L, lo0, log_n, tw)
     for e, g in enumerate(gi):
         if join:
             ja, jb, jo = join
@@ -110,12 +180,11 @@ def pass_tile(dif, data, bx, log_n, s_lo, k, log_L, tw, join=None):
 def mid_tile(data, bx, log_n, k, tw, tw_inv, coset, join=None):
     tile = 1 << k
     base = bx << k
-    sm = data[base:base + tile]
-    for j in range(k - 1, -1, -1):
-        run_stage(True, sm, j, 0, 0, 0, log_n, tile // 2, tw_inv)
-    sm = [(x * coset[base + e]) % R for e, x in enumerate(sm)]
-    for j in range(k):
-        run_stage(False, sm, j, 0, 0, 0, log_n, tile // 2, tw)
+    sm = Tile(data[base:base + tile])
+    run_stages(True, sm, k, 0, 0, 0, log_n, tw_inv)
+    for e in range(tile):
+        sm[e] = sm[e] * coset[base + e]
+    run_stages(False, sm, k, 0, 0, 0, log_n, tw)
     for e in range(tile):
         if join:
             ja, jb, jo = join
@@ -198,7 +267,7 @@ def oracle_icn(log_n, data):
     return [O.from_mont(O.from_bytes(out[32 * i:32 * i + 32])) for i in range(1 << log_n)]
 
 
-def test_every_tiling_gives_the_oracle_intt_coset_ntt(plans):
+def test_every_tiling_gives_the_oracle_intt_coset_ntt(plans, stages):
     # tiles small enough that sizes up to 2^9 take several outer passes, including the
     # uneven splits and the narrowed columns (log_L < outer_log_l) of the lowest pass
     cases = [(t, l, n) for t in range(1, 7) for l in range(0, 6) for n in range(1, 10)]
@@ -222,7 +291,7 @@ def test_every_tiling_gives_the_oracle_intt_coset_ntt(plans):
     assert checked > 100
 
 
-def test_h_pipeline_gives_the_oracle_h(plans):
+def test_h_pipeline_gives_the_oracle_h(plans, stages):
     cases = [(t, l, n) for t, l in ((2, 0), (2, 1), (3, 1), (4, 2), (5, 4), (11, 2)) for n in (1, 2, 5, 8)]
     rng = random.Random(4)
     for (t, l, log_n), plan in zip(cases, plans(cases)):
@@ -232,6 +301,22 @@ def test_h_pipeline_gives_the_oracle_h(plans):
         A, B, C = oracle_icn(log_n, a), oracle_icn(log_n, b), oracle_icn(log_n, c)
         want = [(x * y - z) % R for x, y, z in zip(A, B, C)]
         assert emulate_h_pipeline(plan, log_n, a, b, c, tabs) == want, (t, l, log_n)
+
+
+def test_tile_slots_are_a_permutation_without_bank_conflicts():
+    """Tile::slot moves an element within its 32 and is one to one in tiles of any size;
+    in run_two_stages the 8 lanes of one 128-bit access meet 8 different 16-byte banks."""
+    for k in range(1, 13):
+        assert sorted(map(slot, range(1 << k))) == list(range(1 << k))
+    for log_L in range(5):
+        for k in range(max(2, 5 - log_L), 11 - log_L):
+            quads = (1 << k << log_L) // 4
+            for j in range(0, k - 1):
+                for q0 in range(0, quads - 7, 8):
+                    for i in range(4):
+                        banks = {slot(stage_elements(q, j, log_L, True)[0] + (i << (j + log_L))) % 8
+                                 for q in range(q0, q0 + 8)}
+                        assert len(banks) == 8, (log_L, k, j, i)
 
 
 BATCH_PROBE = r"""
