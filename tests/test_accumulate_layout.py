@@ -1,12 +1,13 @@
-"""The MSM accumulate's chunking and partial-sum layout (msm.cu: chunk_len, k_nseg,
-accumulate_chunks, k_fat_merge_jobs/_final, k_bucket_sums), restated line for
-line on Python integers (a point becomes the integer it stands for, an addition
-a +).  For skewed bucket sizes -- empty buckets, a bucket holding most entries
+"""The MSM accumulate's chunking and partial-sum layout (msm.cu: min_chunk, chunk_len,
+k_plan_sums/_offsets/_segments, accumulate_chunks, k_fat_merge_jobs/_final,
+k_bucket_sums), restated line for line on Python integers (a point becomes the
+integer it stands for, an addition a +).  For skewed bucket sizes -- empty buckets, a bucket holding most entries
 (a witness full of ones), single entries -- every chunk's partial sum lands in
 its own slot of its bucket's range, every slot is written once, the fat-bucket
 jobs and the bucket sums give each bucket the sum of its entries, and the chunk
-length keeps the thread count within its cap.  The GPU parity tests check the
-CUDA code itself."""
+length keeps the thread count within its cap and within the chunks that the
+buffers are sized for (msm_max_chunks, compiled here from msm.cuh).  The GPU parity
+tests check the CUDA code itself."""
 import os
 import random
 import shutil
@@ -17,6 +18,11 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 ACC_THREADS = 1 << 19
 FAT_PARTIALS, FAT_JOBS, FAT_JOB_MIN = 16, 64, 128
+SPREAD_THREADS = 148 * 512
+
+
+def min_chunk(M, floor):
+    return max(floor, min(16, (M + SPREAD_THREADS - 1) // SPREAD_THREADS))
 
 
 def chunk_len(M, K, L_min, wave):
@@ -37,17 +43,42 @@ def fat_job_len(ns):
     return max(FAT_JOB_MIN, (ns + FAT_JOBS - 1) // FAT_JOBS)
 
 
-def layout_and_sums(sizes, values, L):
+def plan(sizes, K, L_floor, wave, tile=1024, per_block=1):
+    """k_plan_sums, k_plan_offsets and k_plan_segments: M, L, the bucket offsets, the
+    partial sums per bucket, their bases and the fat list, block by block."""
     Ks = len(sizes)
-    offsets = [0]
-    for s in sizes:
-        offsets.append(offsets[-1] + s)
-    M = offsets[-1]
-    # k_nseg: partials per bucket; seg_base is their exclusive scan
-    nseg = [((hi - 1) // L - lo // L + 1) if hi > lo else 0 for lo, hi in zip(offsets, offsets[1:])]
-    seg_base = [0]
-    for n in nseg:
-        seg_base.append(seg_base[-1] + n)
+    tiles = (Ks + tile - 1) // tile
+    blocks = max(1, (tiles + per_block - 1) // per_block)
+    mine = lambda b: [range(t * tile, min((t + 1) * tile, Ks))
+                      for t in range(b * per_block, min((b + 1) * per_block, tiles))]
+    sums = [sum(sizes[g] for t in mine(b) for g in t) for b in range(blocks)]
+    M = sum(sums)
+    L = chunk_len(M, K, min_chunk(M, L_floor), wave)
+    offsets, counts, fat = [None] * Ks + [M], [None] * Ks, []
+    psums = [0] * blocks
+    for b in range(blocks):
+        off = sum(sums[:b])
+        for g in (g for t in mine(b) for g in t):
+            assert offsets[g] is None
+            offsets[g], hi = off, off + sizes[g]
+            counts[g] = (hi - 1) // L - off // L + 1 if sizes[g] else 0
+            if g < K and counts[g] > FAT_PARTIALS:
+                fat.append(g)
+            psums[b] += counts[g]
+            off = hi
+    seg_base = [None] * Ks + [sum(psums)]
+    for b in range(blocks):
+        off = sum(psums[:b])
+        for g in (g for t in mine(b) for g in t):
+            seg_base[g] = off
+            off += counts[g]
+    return M, L, offsets, counts, seg_base, fat
+
+
+def layout_and_sums(sizes, values, K, L_floor, wave, tile=1024, per_block=1):
+    Ks = len(sizes)
+    M, L, offsets, nseg, seg_base, fat = plan(sizes, K, L_floor, wave, tile, per_block)
+    assert M == len(values) and None not in offsets and None not in seg_base
     partials = [None] * seg_base[-1]
 
     def store(g, t, acc):
@@ -80,10 +111,9 @@ def layout_and_sums(sizes, values, L):
     assert None not in partials, "a partial slot no chunk wrote"
     # fat buckets: FAT_JOBS jobs of J partials folded into each job's first slot, then
     # the job results (slots base + t J, one thread each) into the first slot
-    for g in range(Ks):
+    assert sorted(fat) == [g for g in range(K) if nseg[g] > FAT_PARTIALS]
+    for g in fat:
         ns, base = nseg[g], seg_base[g]
-        if ns <= FAT_PARTIALS:
-            continue
         J = fat_job_len(ns)
         assert FAT_JOBS * J >= ns
         for j in range(FAT_JOBS):
@@ -91,15 +121,15 @@ def layout_and_sums(sizes, values, L):
             if a < ns:
                 partials[base + a] = sum(partials[base + a:base + min(a + J, ns)])
         partials[base] = sum(partials[base + t * J] for t in range(64) if t * J < ns)
-    # k_bucket_sums
+    # k_bucket_sums, over the real buckets
     return [partials[seg_base[g]] if nseg[g] > FAT_PARTIALS else sum(partials[seg_base[g]:seg_base[g] + nseg[g]])
-            for g in range(Ks)], offsets
+            for g in range(K)], offsets, L
 
 
 def test_chunk_partials_fold_back_to_each_bucket():
     rng = random.Random(21)
     for trial in range(48):
-        K = rng.choice([1, 2, 7, 64, 512, 2048])
+        K = rng.choice([1, 2, 7, 64, 512, 2048, 3000])
         kind = trial % 4
         if kind == 0:     # uniform
             sizes = [rng.randrange(0, 12) for _ in range(K)]
@@ -110,16 +140,75 @@ def test_chunk_partials_fold_back_to_each_bucket():
             sizes = [rng.choice([0, 0, 0, 0, 1, 30]) for _ in range(K)]
         else:             # a few giant buckets
             sizes = [rng.choice([0, 0, 0, 1, 3000]) for _ in range(min(K, 64))]
-        sizes.append(rng.randrange(0, 50))   # the constant-work sink bucket, accumulated, never reduced
+        K = len(sizes)
+        if rng.randrange(2):
+            sizes.append(rng.randrange(0, 2000))   # the constant-work sink bucket, accumulated, never reduced
         M = sum(sizes)
         if M == 0:
             continue
         values = [rng.randrange(1, 1 << 30) for _ in range(M)]
-        L = chunk_len(M, K, 16, rng.choice([0, 148 * 512, 148]))
-        assert L >= 16 and (M + L - 1) // L <= max(ACC_THREADS, 1)
-        sums, offsets = layout_and_sums(sizes, values, L)
-        for g in range(len(sizes)):
+        floor = rng.choice([4, 16])
+        sums, offsets, L = layout_and_sums(sizes, values, K, floor, rng.choice([0, 148 * 512, 148]),
+                                           *rng.choice([(1024, 1), (16, 1), (16, 3), (4, 2)]))
+        assert L >= floor and (M + L - 1) // L <= ACC_THREADS
+        for g in range(K):
             assert sums[g] == sum(values[offsets[g]:offsets[g + 1]]), (trial, g)
+
+
+def test_every_short_chunk_length_folds_back():
+    # 4 to 16 entries a chunk, over buckets that start and end anywhere in one
+    rng = random.Random(22)
+    for L in range(4, 17):
+        sizes = [rng.choice([0, 0, 0, 1, 2, 3, 5, 17, 60]) for _ in range(120)]   # below 4 L a bucket on average
+        values = [rng.randrange(1, 1 << 30) for _ in range(sum(sizes))]
+        sums, offsets, got = layout_and_sums(sizes, values, len(sizes), L, 0)
+        assert got == L
+        assert sums == [sum(values[a:b]) for a, b in zip(offsets, offsets[1:])]
+
+
+def test_min_chunk_cases():
+    # down to the floor while the chunks leave SMs without their 512 threads, 16 from there on
+    assert [min_chunk(M, 4) for M in (0, 1, 4 * SPREAD_THREADS, 4 * SPREAD_THREADS + 1, 15 * SPREAD_THREADS,
+                                      15 * SPREAD_THREADS + 1, 1 << 30)] == [4, 4, 4, 5, 15, 16, 16]
+    assert {min_chunk(M, 16) for M in (0, 1, 1 << 18, 1 << 30)} == {16}
+
+
+CHUNKS_PROBE = r"""
+#include <cstdio>
+#include "msm.cuh"
+int main() {
+    unsigned long long m;
+    unsigned floor;
+    while (scanf("%llu %u", &m, &floor) == 2) printf("%zu\n", g16::msm_max_chunks(m, floor));
+    return 0;
+}
+"""
+
+
+def test_chunks_never_exceed_what_the_buffers_hold(tmp_path):
+    """ceil(M / L) <= msm_max_chunks(max_entries) for every entry count M up to the maximum
+    that a call's buffers and its accumulate launch are sized for."""
+    if shutil.which("nvcc") is None:
+        pytest.skip("nvcc not on PATH")
+    src, exe = tmp_path / "probe.cu", tmp_path / "probe"
+    src.write_text(CHUNKS_PROBE)
+    subprocess.run(["nvcc", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "snarkrs_b200", "csrc"), "-I",
+                    os.path.join(ROOT, "include"), "-o", str(exe), str(src)], check=True, capture_output=True)
+    rng = random.Random(23)
+    edges = [k * SPREAD_THREADS + d for k in (1, 2, 3, 4, 5, 8, 15, 16, 17, 20, 32, 33, 48) for d in (-1, 0, 1)]
+    Ms = sorted(set([0, 1, 3, 4, 5, 15, 16, 17, 1000, 1 << 20, 1 << 26, (1 << 31) - 1] + edges +
+                    [int(1.3 ** rng.uniform(1, 80)) for _ in range(300)]))
+    for floor in (4, 16):
+        out = subprocess.run([str(exe)], input=" ".join("%d %d" % (m, floor) for m in Ms), capture_output=True,
+                             text=True, check=True).stdout.split()
+        most, held = 0, list(map(int, out))
+        for M, cap in zip(Ms, held):
+            assert cap >= most, "a larger maximum never holds fewer chunks"
+            for K in (1, 1000, 1 << 13, 1 << 20):
+                for wave in (0, 148, SPREAD_THREADS):
+                    L = chunk_len(M, K, min_chunk(M, floor), wave)
+                    assert L >= floor and (M + L - 1) // L <= cap, (M, K, floor, wave)
+                    most = max(most, (M + L - 1) // L)
 
 
 def test_chunk_len_cases():
