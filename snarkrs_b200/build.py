@@ -22,7 +22,7 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 SOURCES = ["host_bn254.cpp", "formats.cpp", "gnark.cpp", "synth.cpp", "msm.cu", "msm_noalloc.cu", "ntt.cu", "prover.cu", "batch.cu", "server.cpp", "pairing.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-O3", "-I", CSRC, "-I", os.path.join(ROOT, "include")]
-# extra nvcc flags for experiments (e.g. -DACC_G2_MIN_BLOCKS=3); pass --force when they change
+# extra nvcc flags for experiments (e.g. -DG16_REDUCE_LB_G1=6); pass --force when they change
 EXTRA = os.environ.get("G16_NVCC_EXTRA", "").split()
 
 

@@ -13,12 +13,13 @@
 // GPUs).  Within a vector the partial products a[j] b do not overlap, so a row
 // is one carry chain of 32x32+64-bit multiply-adds and no other instruction;
 // the carry between the vectors rides into the next row's chain.  What bounds
-// it is the issue rate of wide multiply-adds, 32 a clock on an SM: 136 of them
-// a product leave 69.6 G products/s on 148 SMs at 1965 MHz, and it measured
-// 66.5 G/s (one product per thread and step, 1024 threads an SM) and 845
-// cycles for one warp's dependent product, against 44.0 G/s and 1127 cycles
-// for the form it replaced, a single vector whose carries were 64-bit sums on
-// the ALU pipe.
+// it is the issue rate of multiply-adds: 128 wide ones at 32 a clock on an SM
+// and 8 low halves (the quotient digits) at 64 a clock are 4.125 clocks a
+// product, 70.5 G products/s on 148 SMs at 1965 MHz.  It measured 66.5 G/s, 0.94
+// of that (one product per thread and step, 1024 threads an SM), and 845 cycles
+// for one warp's dependent product, against 44.0 G/s and 1127 cycles for the
+// form it replaced, a single vector whose carries were 64-bit sums on the ALU
+// pipe.
 // BN254's moduli are below 2^254, so the running sum stays below 2^287 and
 // fits nine limbs; the carry out of the ninth is provably zero.
 #pragma once
@@ -741,11 +742,12 @@ __device__ __forceinline__ Fq2 sqr(const Fq2& a) {
 }
 
 // ---- product policy: inlined, or one out-of-line copy ----
-// Latency-bound kernels (bucket reduction) run long dependent chains of point
-// operations; inlining ~14 CIOS bodies per point operation, several operations
-// per kernel, overflows the instruction cache.  They call a single
-// out-of-line copy instead (operands by value, so they stay in registers).
-// The throughput kernels keep every product inlined.
+// The G1 accumulate, the NTT and the groups of lanes (lanes.cuh) keep every
+// product inlined.  The G2 accumulate calls one out-of-line Fq2 product
+// (operands by value, so they stay in registers): ten inlined ones overflow the
+// instruction cache (2.44 against 2.18 ms for a 2^18 MSM).  So do the
+// window tables, the key generator and the rare doubling inside an addition,
+// where code size counts and speed does not.
 template <class Params>
 __device__ __noinline__ Fp<Params> mul_ool(Fp<Params> a, Fp<Params> b) {
     return mul(a, b);
@@ -764,9 +766,9 @@ __device__ __forceinline__ Fp<Params> fsqr(const Fp<Params>& a) {
 
 // Out-of-line copies that hold several independent products.  A warp issues
 // in order and a CIOS product is one long carry chain, so a lone out-of-line
-// product leaves the pipe idle for most of its latency; two or three chains in
-// one body are scheduled side by side.  The latency-bound kernels group the
-// independent products of each point formula this way.
+// product leaves the pipe idle for part of its latency; two or three chains in
+// one body are scheduled side by side.  The point formulas over G1 that run out
+// of line (window tables, rare doublings) group their independent products this way.
 template <class F>
 struct Two {
     F a, b;

@@ -2,15 +2,17 @@
 //
 // A point operation is ten to fourteen products deep when one thread runs it,
 // and a warp takes 845 cycles for a dependent product whether one of its lanes
-// works or all 32 (136 wide multiply-adds at 8 lanes a clock: the pipe, not the
-// latency, is what a lone warp waits for).  The reduction's last steps have few
-// points left, so here every point is spread over a group of lanes, one
-// coordinate each (X, Y, ZZ, ZZZ), and the independent products of a formula
-// run side by side: an addition is four products deep and a doubling three.
-// The 14 products of an addition fill 16 slots, so a group's addition costs a
-// full device about a sixth more than a thread's, and a third of the time
-// where warps are few.  A lane holds a quarter of each point: no spills, and
-// 256 threads at under 100 registers where a thread's version needed 250.
+// works or all 32: 528 to issue its multiply-adds (128 wide at 8 lanes a clock,
+// 8 low halves at 16) and about 320 of latency that nothing covers.  The
+// reduction's last steps have few points left, so here every point is spread
+// over a group of lanes, one coordinate each (X, Y, ZZ, ZZZ), and the
+// independent products of a formula run side by side: an addition is four
+// products deep and a doubling three.  The 14 products of an addition fill 16
+// slots, so a group's addition costs a full device about a sixth more than a
+// thread's, and a third of the time where warps are few.  A lane holds a quarter
+// of each point: blocks of 256 threads at 80 to 102 registers over G1 and 100 to
+// 113 over G2, two blocks an SM, where a thread's version needed 250.  Only
+// k_reduce_sets spills over G1 (44 bytes, at 80 registers).
 //
 // A G1 point takes 4 lanes; a G2 point 8, lane 2k + i holding component i of
 // coordinate k.  A group's lanes are consecutive and aligned, and lane q's

@@ -64,10 +64,12 @@ __device__ __forceinline__ void stage_scalar(const uint4* __restrict__ scalars, 
 
 // A block of 256 threads takes 256 / WPG scalars: WPG warps share 32 scalars
 // and split their windows.  One warp per 32 scalars (WPG = 1) keeps every lane
-// busy in the conversion; below DIGITS_SPLIT scalars its blocks leave most of
-// the SMs empty and the serial loop over the windows is what is waited for, so
-// eight warps split it (1000 scalars of 23 windows: digits 19 -> 7 us, scatter
-// 26 -> 9 us).
+// busy in the conversion but runs through the windows alone, waiting for an
+// atomic in each; eight warps wait side by side.  Digits and scatter together,
+// one warp / eight, us (uniform scalars; 70% zeros and ones): 2^10 44 / 17, 38 /
+// 17; 2^14 44 / 26, 36 / 19; 2^16 57 / 46, 35 / 26; 2^17 102 / 82, 56 / 46; 2^18
+// 108 / 104, 57 / 55; 2^19 198 / 198, 86 / 93; 2^20 358 / 364, 145 / 157.  From
+// 2^19 on there are warps enough, and the conversion on one warp in eight costs.
 constexpr uint32_t DIGITS_SPLIT = 1u << 18;
 
 template <int WPG>
@@ -246,8 +248,8 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* warp_t
 constexpr uint32_t FAT_PARTIALS = 16;
 constexpr uint32_t FAT_JOBS = 64;
 
-// partials per job of a fat bucket: at least one per thread of the folding
-// block (FAT_JOB_MIN), at most FAT_JOBS jobs
+// partials per job of a fat bucket: FAT_JOB_MIN or more, two or four for each of
+// the folding block's 64 (G1) or 32 (G2) groups of lanes, at most FAT_JOBS jobs
 constexpr uint32_t FAT_JOB_MIN = 128;
 __device__ __forceinline__ uint32_t fat_job_len(uint32_t ns) {
     uint32_t j = (ns + FAT_JOBS - 1) / FAT_JOBS;
@@ -262,7 +264,11 @@ __device__ __forceinline__ uint32_t fat_job_len(uint32_t ns) {
 // over the whole GPU.  Last, the chunks are fitted to whole waves of `wave`
 // threads (the G1 accumulate's 512 threads an SM) when that saves 5% or more: a
 // launch takes about (waves x L) additions per thread, so 2.4 waves of 16
-// entries lose to 2 waves of 20 (a sparse witness MSM of the 2^21 prove).
+// entries lose to 2 waves of 20 (a sparse witness MSM of the 2^21 prove).  A
+// sort that only a G2 accumulate reads is fitted to the same wave although that
+// kernel holds 384 threads an SM: G2 MSMs with a wave of 512 / 384 / no fitting,
+// us: 2^18 uniform 3520 / 3570 / 3560, 200007 2993 / 2994 / 3068, 100003 1998 /
+// 2010 / 2048, 2^17 sparse 1448 / 1403 / 1446; neither wins throughout.
 constexpr uint32_t ACC_THREADS = 1u << 19;
 
 __device__ __forceinline__ uint32_t chunk_len(uint32_t M, uint32_t K, uint32_t L_min, uint32_t wave) {
@@ -438,10 +444,13 @@ struct MsmSegDev {
 };
 
 // ---- accumulate: one thread per chunk of L sorted entries ----
-// Bound by the issue of wide multiply-adds (1232 for a G1 mixed addition, 3200
-// for a G2 one): 6.7 G G1 additions/s in a 2^20 MSM, 0.89 of the rate at which
-// an SM issues them.  Warps run freely; a block-wide barrier after every entry,
-// which kept a longer body in the instruction cache, costs 12% now.
+// Bound by the issue of multiply-adds.  A G1 mixed addition takes 1160 wide ones
+// and 72 low halves at half their cost, 1196 in all, a G2 one 3072 and 160, 3152
+// (eight products of 320 + 16 and two squares of 256 + 16): at 32 a clock on an
+// SM at most 7.78 and 2.95 G additions/s.  Measured 6.7 over G1 (2^20 and 2^21
+// MSMs), 0.86 of that, and 2.2 over G2, 0.76, where 392 bytes of spills and 12
+// warps an SM leave the pipe idle.  Warps run freely; a block-wide barrier after
+// every entry, which kept a longer body in the instruction cache, costs 12% now.
 // MULTI: the buckets belong to several MSMs (segments, msm_space_*), each
 // with its own base table; the segment of bucket g is the last one whose
 // key_start is <= g, followed forward as g grows.
@@ -1234,9 +1243,14 @@ cudaError_t msm_window_table_g2(const void* d_in, size_t n, uint32_t skip, int c
 }
 
 int msm_window_bits(size_t m) {
-    // cost ~ windows * (m + 3.75 * buckets), a bucket at about four mixed additions
-    // (measured: 2^16 points 637 us at 12 bits, 699 at 13 and 14; 2^18 1330 at 15,
-    // 1472 at 13, 1517 at 16; 2^20 3690 at 16, 3625 at 15, 3895 at 17)
+    // cost ~ windows * (m + 3.75 * buckets), a bucket at about four mixed additions.
+    // us by width, the model's choice in brackets, G1: 2^14 9: 389, [10: 416], 11:
+    // 450; 2^16 11: 643, [12: 629], 13: 690; 2^17 12: 891, [13: 939], 14: 937; 2^18
+    // 14: 1394, [15: 1326], 16: 1513; 2^20 15: 3625, [16: 3692], 17: 3894.  G2: 2^14
+    // 9: 905, [10: 903], 11: 1012; 2^16 11: 1596, [12: 1589], 13: 1641; 2^18 14: 3613,
+    // [15: 3522], 16: 4074.  A step to either side is at most 7% better (2^14).  For
+    // scalars of which 70% are 0 or 1 it is one to three bits too wide, since it
+    // counts all of them: 2^18 836 at 15 bits, 719 at 12.
     int best = 8;
     double best_cost = 1e300;
     for (int c = 8; c <= 18; c++) {

@@ -23,9 +23,9 @@
 //   5. the reduction sum_b (b+1) S_b: pieces of seg buckets are folded by
 //      running sums, blocks split the pieces' weights over their bits in
 //      shared memory (msm_reduce_plan), a second kernel sums the blocks' bit
-//      terms per set, a third forms each set's sum; no step has a long dependent chain, and every point
-//      operation is spread over a group of lanes (lanes.cuh), since a
-//      dependent XYZZ addition costs microseconds of latency;
+//      terms per set, a third forms each set's sum; no step has a long
+//      dependent chain, and every point operation is spread over a group of
+//      lanes (lanes.cuh), since a dependent XYZZ addition costs microseconds;
 //   6. host: Horner over the W window sums (c doublings between windows).
 // One sort serves every base vector that shares the scalars: the prover
 // sorts the witness once and accumulates A, B1, L (G1) and B2 (G2) from it.
@@ -40,20 +40,22 @@ namespace g16 {
 
 // Bucket reduction plan for `sets` bucket sets of B buckets each (B a power of
 // two).  A set's sum is sum_b (b + 1) S_b.  Its buckets are cut into pieces of
-// seg buckets (one thread's running sums), 2^lb pieces per block (lb =
-// MSM_REDUCE_LB_G1 or _G2 below; a block keeps two arrays of 2^lb points in
-// shared memory), nb = 2^hb blocks per set.  Each block leaves lb + 2 points, T, G_0 .. G_(lb-1)
-// and its run total R; with more than two blocks in all, a second kernel sums
+// seg buckets (two groups of lanes each, one per running sum), 2^lb pieces per
+// block (lb = MSM_REDUCE_LB_G1 or _G2 below; a block keeps two arrays of 2^lb
+// points in shared memory), nb = 2^hb blocks per set.  Each block leaves lb + 2
+// points, T, G_0 .. G_(lb-1) and its run total R; with more than two blocks in all, a second kernel sums
 // them per set into lb + 1 + hb points, T, G_0 .. G_(lb-1), Gb_0 .. Gb_(hb-1),
 // and the last one forms, one block per set,
 //   set sum = T + seg (sum_j 2^j G_j + 2^lb sum_i 2^i Gb_i).
 // seg grows (up to 32) until the pieces over all sets number at most the
 // target.  Fewer, longer pieces keep the reduction's footprint small where it
 // runs beside other MSMs' accumulations: the prover's window-shifted MSMs (one
-// bucket set) aim at 8192 pieces, 512 threads an SM over G1.  A standalone MSM
+// bucket set) aim at 8192 pieces, 443 threads an SM over G1.  A standalone MSM
 // (one set per window) has the GPU to itself and aims at 32768, shortening the
 // chains; so does the prover's H MSM (MsmSort::reduce_pieces), whose reduction
-// runs last, when the witness MSMs' accumulations are mostly done.
+// runs last, when the witness MSMs' accumulations are mostly done.  Both targets
+// were swept with one thread a piece (the 2^21-constraint prove 45.7 proofs/s at
+// 8192 against 44.1 at 32768) and not again with groups of lanes.
 constexpr uint64_t MSM_REDUCE_PIECES = 8192;
 constexpr uint64_t MSM_REDUCE_PIECES_ALONE = 32768;
 constexpr uint32_t MSM_REDUCE_MAX_SEG = 32;
@@ -152,7 +154,9 @@ inline MsmSpaceReduceLayout msm_space_reduce_layout(const std::vector<uint32_t>&
 // MSM_MIN_CHUNK when that would leave SMs without their 512 threads (min_chunk
 // in msm.cu).  Buffers hold the most chunks any entry count up to the maximum
 // can give: up to 58 MB more for a proof with the smaller floor, which a device
-// memory budget without room for it keeps off (MsmSort::chunk_floor).
+// memory budget without room for it keeps off (MsmSort::chunk_floor).  The
+// spread is a constant, a B200's 148 SMs, because buffers are sized on the host
+// by the same arithmetic as the kernels use.
 constexpr uint32_t MSM_CHUNK = 16;
 constexpr uint32_t MSM_MIN_CHUNK = 4;
 constexpr uint32_t MSM_SPREAD_THREADS = 148 * 512;
@@ -223,8 +227,8 @@ struct MsmAccum {
     void release();
 };
 
-// Window width for m scalars that reach the buckets.  The reference CPU model
-// (crates/msm/src/lib.rs:160-172) with the GPU's cheaper bucket reduction.
+// Window width for m scalars that reach the buckets: the reference CPU model
+// (crates/msm/src/lib.rs:160-172) with what a bucket costs here.
 int msm_window_bits(size_t m);
 
 // Sort n device-resident scalars (32 bytes each; montgomery != 0 converts

@@ -27,9 +27,9 @@ namespace g16 {
 // elements with k <= tile_log - outer_log_l (2^outer_log_l consecutive
 // columns per tile row).  The values are the same for every tiling; only the
 // number of passes over HBM and the shared-memory footprint change.
-struct NttTiling {
-    uint32_t tile_log = 9;       // 512 elements, 16 KiB of shared memory
-    uint32_t outer_log_l = 3;    // 8 columns = 256-byte rows
+struct NttTiling {   // ntt_tables sets a transform's by its size (ntt_default_tiling)
+    uint32_t tile_log = 8;       // 2^tile_log elements of 32 bytes in shared memory
+    uint32_t outer_log_l = 2;    // rows of 2^outer_log_l columns, 32 bytes each
 };
 constexpr uint32_t NTT_MAX_TILE_LOG = 12;   // 128 KiB of shared memory
 
