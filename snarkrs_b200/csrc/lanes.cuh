@@ -10,9 +10,8 @@
 // products deep and a doubling three.  The 14 products of an addition fill 16
 // slots, so a group's addition costs a full device about a sixth more than a
 // thread's, and a third of the time where warps are few.  A lane holds a quarter
-// of each point: blocks of 256 threads at 80 to 102 registers over G1 and 100 to
-// 113 over G2, two blocks an SM, where a thread's version needed 250.  Only
-// k_reduce_sets spills over G1 (44 bytes, at 80 registers).
+// of each point: blocks of 256 threads at 95 to 106 registers over G1 and 100 to
+// 122 over G2, two blocks an SM and no spills, where a thread's version needed 250.
 //
 // A G1 point takes 4 lanes; a G2 point 8, lane 2k + i holding component i of
 // coordinate k.  A group's lanes are consecutive and aligned, and lane q's
@@ -98,10 +97,22 @@ struct Place {
     }
 };
 
+// Bit 2 C of each group of a warp (the lane of ZZ's first component), and those
+// bits where the group's point is the identity, from a warp's ballot of zero
+// elements: the same value in every lane.
+template <class F>
+constexpr unsigned ZZ_LANES = Lanes<F>::C == 1 ? 0x44444444u : 0x10101010u;
+template <class F>
+__device__ __forceinline__ unsigned identities(unsigned ballot) {
+    return (Lanes<F>::C == 1 ? ballot : ballot & (ballot >> 1)) & ZZ_LANES<F>;
+}
+
 // 2 p (dbl-2008-s-1): V = (2Y)^2 and X^2; then W = 2Y V, S = X V, ZZ3 = V ZZ and
-// M^2; then M (S - X3), W Y and ZZZ3 = W ZZZ.  The identity stays itself.
+// M^2; then M (S - X3), W Y and ZZZ3 = W ZZZ.  The identity stays itself; a warp
+// of identities returns at once.
 template <class F>
 __device__ __forceinline__ Fq lanes_dbl(const Fq& p) {
+    if (identities<F>(__ballot_sync(FULL_WARP, p.is_zero())) == ZZ_LANES<F>) return p;
     const Place<F> g;
     const Fq u = pick(g.k == 1, dbl(p), p);
     const Fq s1 = lane_mul<F>(u, u);                     // k 0: X^2, 1: V
@@ -119,13 +130,19 @@ __device__ __forceinline__ Fq lanes_dbl(const Fq& p) {
 
 // p + q (add-2008-s), the identity and equal operands included: U1, S1, U2, S2;
 // then P^2, R^2, ZZ1 ZZ2, ZZZ1 ZZZ2; then Q, PPP, ZZ3; then R (Q - X3), S1 PPP
-// and ZZZ3.  p + (-p) comes out with ZZ3 = ZZZ3 = 0, the identity.
+// and ZZZ3.  p + (-p) comes out with ZZ3 = ZZZ3 = 0, the identity.  A warp whose
+// groups each have an identity operand forms no product: the reduction of few or
+// no full buckets costs little (MSMs with every scalar zero, G1 2^20 638 us with
+// the products and 217 without, G2 2^18 880 and 167; every scalar one, 899 and
+// 479, 1207 and 502; uniform ones level).
 template <class F>
 __device__ __forceinline__ Fq lanes_add(const Fq& p, const Fq& q) {
     constexpr int C = Lanes<F>::C;
     const Place<F> g;
-    const bool p_inf = g.zero(__ballot_sync(FULL_WARP, p.is_zero()), 2);
-    const bool q_inf = g.zero(__ballot_sync(FULL_WARP, q.is_zero()), 2);
+    const unsigned pz = __ballot_sync(FULL_WARP, p.is_zero()), qz = __ballot_sync(FULL_WARP, q.is_zero());
+    const bool p_inf = g.zero(pz, 2);
+    if ((identities<F>(pz) | identities<F>(qz)) == ZZ_LANES<F>) return pick(p_inf, q, p);
+    const bool q_inf = g.zero(qz, 2);
     const Fq t = lane_mul<F>(p, shfl_xor(q, 2 * C));     // U1, S1, U2, S2
     const Fq tx = shfl_xor(t, 2 * C);
     const bool low = g.k < 2;

@@ -447,9 +447,9 @@ struct MsmSegDev {
 // Bound by the issue of multiply-adds.  A G1 mixed addition takes 1160 wide ones
 // and 72 low halves at half their cost, 1196 in all, a G2 one 3072 and 160, 3152
 // (eight products of 320 + 16 and two squares of 256 + 16): at 32 a clock on an
-// SM at most 7.78 and 2.95 G additions/s.  Measured 6.7 over G1 (2^20 and 2^21
-// MSMs), 0.86 of that, and 2.2 over G2, 0.76, where 392 bytes of spills and 12
-// warps an SM leave the pipe idle.  Warps run freely; a block-wide barrier after
+// SM at most 7.78 and 2.95 G additions/s.  Measured 6.7 to 6.8 over G1 (MSMs of
+// 2^20 to 2^22), 0.87 of that, and 2.2 over G2, 0.76, where 392 bytes of spills
+// and 12 warps an SM leave the pipe idle.  Warps run freely; a block-wide barrier after
 // every entry, which kept a longer body in the instruction cache, costs 12% now.
 // MULTI: the buckets belong to several MSMs (segments, msm_space_*), each
 // with its own base table; the segment of bucket g is the last one whose

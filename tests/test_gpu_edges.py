@@ -100,3 +100,24 @@ def test_millions_of_buckets(S, O, constant_work):
     c.close()
     b.close()
     ok.close()
+
+
+@pytest.mark.parametrize("group", [1, 2])
+def test_empty_buckets_cost_little(S, backend, group):
+    """A warp of lane groups that only meets identities forms no product: the pieces kernel
+    takes a small part of its time on full buckets (with the products, the same time)."""
+    n = 1 << (18 if group == 1 else 16)
+    bases, msm = _tiled(S, group, n, 1 << 10), S.CudaMsm(backend)
+    run = msm.msm_g1 if group == 1 else msm.msm_g2
+    ms = {}
+    for name, scalars in (("full", S.synth_scalars(3, n, 0)), ("empty", bytes(32 * n))):
+        got = run(bases, scalars)
+        S.kernel_timing(True)
+        S.kernel_timing_reset()
+        try:
+            assert run(bases, scalars) == got
+            ms[name] = S.kernel_timing_report()["msm_reduce"][0]
+        finally:
+            S.kernel_timing(False)
+    assert got == bytes(64 * group)
+    assert ms["empty"] < 0.5 * ms["full"], ms
