@@ -83,6 +83,7 @@ static BatchKey key_of(const g16_circuit* c) {
 struct BatchEngine {
     std::vector<BatchKey> key;              // the layout built; empty: none
     uint64_t accounted = 0;                 // device bytes counted against the backend's budget
+    bool tight = false;                     // the last layout had no room for short accumulate chunks
     void* d_arena = nullptr;
     size_t cap_arena = 0;
     std::vector<size_t> off_w, off_abc, off_h;
@@ -448,18 +449,20 @@ struct BatchUsers {
 // Layout E for the batch, its grow-only buffers counted against the backend's
 // device budget; on failure E keeps no layout.  The accumulates' chunks go below
 // MSM_CHUNK entries where the engine already holds the larger scratch, or where
-// it has to grow anyway and the budget has room for every engine's; so the
-// larger scratch refuses no batch that fits with chunks of MSM_CHUNK, and an
-// engine sized for a batch never grows for it.
+// the budget has room for every engine's; so the larger scratch refuses no batch
+// that fits with chunks of MSM_CHUNK.  An engine that was laid out without it
+// keeps to that until it has to grow: what was sized for a batch never grows for
+// it, even if memory has come free since.
 int layout_engine(g16_backend* b, BatchEngine& E, g16_circuit* const* cs, size_t count) {
     uint64_t need = plan_estimate(cs, count, MSM_CHUNK);
     const uint64_t spread = plan_estimate(cs, count, MSM_MIN_CHUNK);
     uint32_t floor = MSM_CHUNK;
-    if (spread <= E.accounted ||
-        (need > E.accounted && b->vram_used + batch_max_engines() * spread <= b->vram_limit)) {
+    if (spread <= E.accounted || ((!E.tight || need > E.accounted) &&
+                                  b->vram_used + batch_max_engines() * spread <= b->vram_limit)) {
         floor = MSM_MIN_CHUNK;
         need = spread;
     }
+    E.tight = floor == MSM_CHUNK;
     for (MsmSpace* sp : {&E.g1, &E.g2, &E.hs}) sp->sort.chunk_floor = floor;
     if (need > E.accounted) {   // the engine's buffers grow: check and count the difference
         if (b->vram_used + (need - E.accounted) > b->vram_limit)

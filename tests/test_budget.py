@@ -72,3 +72,20 @@ def test_short_chunks_do_not_refuse_a_batch(backend):
     c.close()
     b.close()
     circ.close()
+
+
+@pytest.mark.gpu
+def test_an_engine_with_room_keeps_short_chunks(backend):
+    """An engine that holds enough for a larger mix with chunks of 16 entries still grows to
+    its short chunks' scratch where the budget has room, and then holds it."""
+    sc, zk = _key(3000)
+    b = S.CudaBackend(0)
+    c = b.prepare(S.ProvingKey.from_bytes(zk))
+    one = S.fr_to_mont_bytes(1)
+    job, used = (c, sc.witness(1), one, one), []
+    for n in (4, 5, 5):   # a job's share is below the short chunks' 39 MB
+        b.prove_batch([job] * n)
+        used.append(b.vram_used())
+    assert used[0] < used[1] == used[2]
+    c.close()
+    b.close()
